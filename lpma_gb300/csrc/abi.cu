@@ -1555,7 +1555,7 @@ lpma_status_t lpma_edge_query(LpmaHandle *h, const uint64_t *d_keys, size_t n, u
     if (h->gp) return LPMA_ERR_INVALID_ARGUMENT;  // not offered for the flat GPMA layout
     if (h->sticky != LPMA_OK) return h->sticky;
     if (!n) return LPMA_OK;
-    launch_edge_query(d_keys, (uint32_t)n, window, Geo{h->c.keys, h->c.vals, h->H}, h->c.cnt, h->c.fl, h->sent, h->V,
+    launch_edge_query(d_keys, (uint32_t)n, window, Geo{h->c.keys, h->c.vals, h->H}, h->c.fl, h->sent, h->V,
                       d_counts, (cudaStream_t)stream);
     CK(cudaGetLastError());
     mark_done(h, (cudaStream_t)stream);

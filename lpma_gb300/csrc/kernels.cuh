@@ -158,8 +158,8 @@ void launch_nbr_count(const uint32_t *srcs, const uint64_t *windows, uint32_t n,
 void launch_nbr_fill(const uint32_t *srcs, const uint64_t *windows, uint32_t n, Geo g, const uint8_t *cnt,
                      const uint32_t *sent, uint32_t V, const uint32_t *offsets, uint32_t *nbrs, uint8_t *vals,
                      cudaStream_t s);
-void launch_edge_query(const uint64_t *q, uint32_t n, uint32_t window, Geo g, const uint8_t *cnt,
-                       const ulonglong2 *fl, const uint32_t *sent, uint32_t V, uint32_t *res, cudaStream_t s);
+void launch_edge_query(const uint64_t *q, uint32_t n, uint32_t window, Geo g, const ulonglong2 *fl,
+                       const uint32_t *sent, uint32_t V, uint32_t *res, cudaStream_t s);
 void launch_bfs_init(const uint32_t *sources, uint32_t n, uint32_t V, int32_t *dist, uint32_t *frontier,
                      uint32_t *count, cudaStream_t s);
 void launch_bfs_expand(const uint32_t *frontier, const uint32_t *nf, uint32_t nf_host, int32_t level, Geo g,

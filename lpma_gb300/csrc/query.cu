@@ -144,10 +144,22 @@ __global__ void __launch_bounds__(TPB) k_nbr_fill(const uint32_t *__restrict__ s
 // For key (src, dst, t): the number of stored keys (src, dst, t') with
 // t - window <= t' <= t (the edge-query check of test.cu:46-62; window =
 // 0xFFFFF with t = 0xFFFFF gives check_edge_kernel's any-time test,
-// rpma.cuh:2040-2066).  Binary search over src's segments for the first
-// segment whose last key reaches (src, dst, lb), then a forward count.
+// rpma.cuh:2040-2066).  One thread a query: src's sentinels give its segment
+// range, a binary search over the segments' last keys the first one that
+// reaches (src, dst, lb), five probes of that segment its first key >= lb,
+// and the count goes forward from there.  The sentinel of src ends both
+// searches (it is above every key asked for), so neither tests a bound.
+//
+// Bound by its random reads (sentinels, segment bounds out of L2, slots out
+// of DRAM), about 10 sectors a query.  The segment's bounds stand for its
+// count (an empty one has no first key): one load a step where there were
+// two; the slots are halved twice and a quarter (64 bytes, one DRAM access)
+// loads at once, where they were walked from the first on.  2M queries of a
+// 15M-key graph 184 -> 144 us, 400K of 19M keys 60 -> 39, 4K 21 -> 13.
+// Measured slower: three probes a step of the segment search (159 us for
+// 2M: more L2 sectors), the three quarter bounds of a segment at once (178:
+// more DRAM accesses).
 __global__ void __launch_bounds__(TPB) k_edge_query(const uint64_t *__restrict__ q, uint32_t n, uint32_t window, Geo g,
-                                                    const uint8_t *__restrict__ cnt,
                                                     const ulonglong2 *__restrict__ fl,
                                                     const uint32_t *__restrict__ sent, uint32_t V, uint32_t *res) {
     for (uint64_t i = blockIdx.x * (uint64_t)TPB + threadIdx.x; i < n; i += gridDim.x * (uint64_t)TPB) {
@@ -160,47 +172,51 @@ __global__ void __launch_bounds__(TPB) k_edge_query(const uint64_t *__restrict__
             const uint32_t lb = t > window ? t - window : 0;
             const uint64_t pre = key & ~TIME_MASK;
             const uint64_t lo = pre | lb, hi = pre | t;
-            uint64_t p0, p1;
-            vertex_range(sent, src, g.H, p0, p1);
-            if (p1 > p0) {
-                const uint64_t S0 = p0 >> 5, S1 = (p1 - 1) >> 5;
-                // first non-empty segment in [S0, S1] whose last key >= lo
-                uint64_t L = S0, R = S1 + 1, ans = S1 + 1;
-                while (L < R) {
-                    const uint64_t mid = (L + R) >> 1;
-                    uint64_t ms = mid;
-                    while (ms < R && cnt[ms] == 0) ms++;
-                    if (ms == R) {
-                        R = mid;
-                        continue;
-                    }
-                    const uint64_t last = fl[heap_of_linear(ms, g.H)].y;
-                    if (last >= lo) {
-                        ans = ms;
-                        R = mid;
-                    } else {
-                        L = ms + 1;
-                    }
+            const uint32_t e1 = sent[src], e0 = src ? sent[src - 1] : 0u;
+            // src's keys lie in the segments of its predecessor's sentinel to its own
+            uint32_t L = src ? (uint32_t)(linear_slot(e0, g.H) >> 5) : 0u;
+            const uint32_t last_seg = (uint32_t)(linear_slot(e1, g.H) >> 5);
+            // first non-empty segment whose last key >= lo (last_seg is one)
+            uint32_t U = last_seg, s = last_seg;
+            while (L < U) {
+                const uint32_t mid = (L + U) >> 1;
+                uint32_t ms = mid;
+                ulonglong2 b = fl[heap_of_linear32(ms, g.H)];
+                while (b.x == KEY_NONE && ++ms < U) b = fl[heap_of_linear32(ms, g.H)];
+                if (ms == U) {
+                    U = mid;  // [mid, U) holds nothing
+                } else if (b.y >= lo) {
+                    s = ms;
+                    U = mid;
+                } else {
+                    L = ms + 1;
                 }
-                bool done = false;
-                for (uint64_t s = ans; s <= S1 && !done; s++) {
-                    const uint32_t c = cnt[s];
-                    const uint64_t j = heap_of_linear(s, g.H);
-                    for (uint32_t l = 0; l < c; l++) {
-                        const uint64_t pos = 32 * s + l;
-                        if (pos < p0) continue;
-                        if (pos >= p1) {
-                            done = true;
-                            break;
-                        }
-                        const uint64_t kk = g.keys[32 * j + l];
-                        if (kk > hi) {
-                            done = true;
-                            break;
-                        }
-                        if (kk >= lo && g.vals[32 * j + l] != VAL_TOMB) found++;
-                    }
+            }
+            const uint64_t *sk = g.keys + 32ull * heap_of_linear32(s, g.H);
+            // the first key >= lo: two probes choose a quarter of the segment,
+            // whose 8 keys (64 bytes) then load together
+            uint32_t pos = sk[15] < lo ? 16u : 0u;
+            if (sk[pos + 7] < lo) pos += 8;
+            {
+                const ulonglong2 *qp = reinterpret_cast<const ulonglong2 *>(sk + pos);
+                const ulonglong2 a = qp[0], b = qp[1], c = qp[2], d = qp[3];
+                pos += (a.x < lo) + (a.y < lo) + (b.x < lo) + (b.y < lo) + (c.x < lo) + (c.y < lo) + (d.x < lo) +
+                       (d.y < lo);
+            }
+            for (;;) {
+                const uint64_t kk = pos < 32 ? sk[pos] : KEY_NONE;
+                if (kk == KEY_NONE) {  // the segment's keys end: the next one that has any
+                    uint64_t first = KEY_NONE;
+                    while (s < last_seg && first == KEY_NONE) first = fl[heap_of_linear32(++s, g.H)].x;
+                    if (first > hi) break;
+                    sk = g.keys + 32ull * heap_of_linear32(s, g.H);
+                    pos = 0;
+                    continue;
                 }
+                if (kk > hi) break;
+                if (g.vals[(uint64_t)(sk - g.keys) + pos] != VAL_TOMB) found++;
+                if (kk == hi) break;  // keys are distinct
+                pos++;
             }
         }
         res[i] = found;
@@ -359,10 +375,10 @@ void launch_nbr_fill(const uint32_t *srcs, const uint64_t *windows, uint32_t n, 
     note_launch();
 }
 
-void launch_edge_query(const uint64_t *q, uint32_t n, uint32_t window, Geo g, const uint8_t *cnt,
-                       const ulonglong2 *fl, const uint32_t *sent, uint32_t V, uint32_t *res, cudaStream_t s) {
+void launch_edge_query(const uint64_t *q, uint32_t n, uint32_t window, Geo g, const ulonglong2 *fl,
+                       const uint32_t *sent, uint32_t V, uint32_t *res, cudaStream_t s) {
     ProfScope ps_("edge_query", s);
-    k_edge_query<<<grid_for(n, TPB, 152 * 16), TPB, 0, s>>>(q, n, window, g, cnt, fl, sent, V, res);
+    k_edge_query<<<grid_for(n, TPB, 152 * 16), TPB, 0, s>>>(q, n, window, g, fl, sent, V, res);
     note_launch();
 }
 
