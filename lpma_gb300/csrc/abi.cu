@@ -136,7 +136,9 @@ struct LpmaHandle {
     // read paths (neighbour query, BFS, PageRank)
     uint32_t *q_cnt = nullptr, *q_tmp = nullptr;
     size_t q_cap = 0;
-    uint32_t *bfs_a = nullptr, *bfs_b = nullptr, *bfs_cnt = nullptr;
+    uint2 *bfs_a = nullptr, *bfs_b = nullptr;  // frontier lists
+    uint32_t *bfs_cnt = nullptr;               // BFS_WORDS counters
+    size_t bfs_cap = 0;
     uint32_t *pr_deg = nullptr;
     double *pr_contrib = nullptr, *pr_acc = nullptr, *pr_dangling = nullptr;
     uint32_t *pin_word = nullptr;  // pinned: totals read back by the read paths
@@ -152,6 +154,12 @@ struct LpmaHandle {
 };
 
 namespace {
+
+// levels of a BFS launched before the host reads their counters back, the
+// counters of those levels (ranges and vertices of each frontier), and the
+// words of the read paths' pinned buffer
+constexpr uint32_t BFS_LEVELS = 4, BFS_WORDS = 2 * (BFS_LEVELS + 1), PIN_WORDS = 16;
+static_assert(BFS_WORDS <= PIN_WORDS, "the counters fit the pinned words");
 
 #define CK(x)                                         \
     do {                                              \
@@ -1205,7 +1213,7 @@ lpma_status_t lpma_destroy(LpmaHandle *h) {
         dfree_async(h->bfs_cnt);
     dfree_async(h->pr_deg), dfree_async(h->pr_contrib), dfree_async(h->pr_acc), dfree_async(h->pr_dangling);
     if (h->done_ev) cudaEventDestroy(h->done_ev);
-    pinned_release(h->pin_word, 2 * sizeof(uint32_t));
+    pinned_release(h->pin_word, PIN_WORDS * sizeof(uint32_t));
     delete h;
     return LPMA_OK;
 }
@@ -1522,7 +1530,7 @@ lpma_status_t lpma_query_neighbors(LpmaHandle *h, const uint32_t *d_srcs, const 
     if (n >= (1u << 30)) return LPMA_ERR_INVALID_ARGUMENT;
     if (h->sticky != LPMA_OK) return h->sticky;
     cudaStream_t s = (cudaStream_t)stream;
-    if (!h->pin_word) CK(pinned_alloc(&h->pin_word, 2 * sizeof(uint32_t)));
+    if (!h->pin_word) CK(pinned_alloc(&h->pin_word, PIN_WORDS * sizeof(uint32_t)));
     if (n > h->q_cap) {
         dfree(h->q_cnt), dfree(h->q_tmp);
         h->q_cap = 0;
@@ -1568,30 +1576,46 @@ lpma_status_t lpma_bfs(LpmaHandle *h, const uint32_t *d_sources, size_t n_source
     if (h->gp) return LPMA_ERR_INVALID_ARGUMENT;  // not offered for the flat GPMA layout
     if (h->sticky != LPMA_OK) return h->sticky;
     cudaStream_t s = (cudaStream_t)stream;
-    if (!h->pin_word) CK(pinned_alloc(&h->pin_word, 2 * sizeof(uint32_t)));
-    if (!h->bfs_a) {
-        CK(dalloc(&h->bfs_a, h->V));
-        CK(dalloc(&h->bfs_b, h->V));
-        CK(dalloc(&h->bfs_cnt, 2));
+    if (!h->pin_word) CK(pinned_alloc(&h->pin_word, PIN_WORDS * sizeof(uint32_t)));
+    const uint32_t cap = bfs_items_for(h->V, h->H);
+    if (cap > h->bfs_cap) {
+        dfree(h->bfs_a), dfree(h->bfs_b);
+        h->bfs_cap = 0;
+        CK(dalloc(&h->bfs_a, cap));
+        CK(dalloc(&h->bfs_b, cap));
+        h->bfs_cap = cap;
     }
-    CK(cudaMemsetAsync(h->bfs_cnt, 0, 2 * sizeof(uint32_t), s));
-    launch_bfs_init(d_sources, (uint32_t)n_sources, h->V, d_dist, h->bfs_a, h->bfs_cnt, s);
-    CK(cudaMemcpyAsync(h->pin_word, h->bfs_cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    CK(host_wait(s, blocking_waits(h)));
-    uint32_t nf = h->pin_word[0], lv = 0;
-    uint64_t total = nf;
-    uint32_t *cur = h->bfs_a, *nxt = h->bfs_b;
+    if (!h->bfs_cnt) CK(dalloc(&h->bfs_cnt, BFS_WORDS));
+    // the frontier's ranges and vertices at the levels of a round
+    uint32_t *items = h->bfs_cnt, *found = h->bfs_cnt + BFS_LEVELS + 1;
     const Geo g{h->c.keys, h->c.vals, h->H};
-    while (nf > 0 && (max_depth == 0 || lv < max_depth)) {
-        CK(cudaMemsetAsync(h->bfs_cnt + 1, 0, sizeof(uint32_t), s));
-        launch_bfs_expand(cur, h->bfs_cnt, nf, (int32_t)lv, g, h->c.cnt, h->sent, d_dist, nxt, h->bfs_cnt + 1, s);
-        CK(cudaMemcpyAsync(h->bfs_cnt, h->bfs_cnt + 1, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-        CK(cudaMemcpyAsync(h->pin_word, h->bfs_cnt + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemsetAsync(h->bfs_cnt, 0, BFS_WORDS * sizeof(uint32_t), s));
+    launch_bfs_init(d_sources, (uint32_t)n_sources, h->V, g, h->sent, d_dist, h->bfs_a, cap, items, found, s);
+    uint2 *cur = h->bfs_a, *nxt = h->bfs_b;
+    uint32_t lv = 0;
+    uint64_t total = 0;
+    // rounds of up to BFS_LEVELS levels, one read-back each (a level whose
+    // frontier turned out empty does nothing)
+    for (uint32_t round = 0;; round++) {
+        const uint32_t k = max_depth ? std::min(BFS_LEVELS, max_depth - lv) : BFS_LEVELS;
+        for (uint32_t j = 0; j < k; j++) {
+            launch_bfs_expand(cur, items + j, (int32_t)(lv + j), g, h->c.cnt, h->sent, d_dist, nxt, cap, items + j + 1,
+                              found + j + 1, s);
+            std::swap(cur, nxt);
+        }
+        CK(cudaMemcpyAsync(h->pin_word, h->bfs_cnt, BFS_WORDS * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         CK(host_wait(s, blocking_waits(h)));
-        nf = h->pin_word[0];
-        total += nf;
-        lv++;
-        std::swap(cur, nxt);
+        const uint32_t *hf = h->pin_word + BFS_LEVELS + 1;
+        if (round == 0) total = hf[0];
+        uint32_t done = 0;
+        while (done < k && hf[done] > 0) total += hf[++done];
+        lv += done;
+        if (done < k || hf[k] == 0 || (max_depth && lv >= max_depth)) break;
+        // the last frontier is the next round's first
+        CK(cudaMemcpyAsync(items, items + k, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+        CK(cudaMemsetAsync(items + 1, 0, BFS_LEVELS * sizeof(uint32_t), s));
+        CK(cudaMemcpyAsync(found, found + k, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+        CK(cudaMemsetAsync(found + 1, 0, BFS_LEVELS * sizeof(uint32_t), s));
     }
     if (levels) *levels = lv;
     if (reached) *reached = total;
@@ -1664,7 +1688,7 @@ lpma_status_t lpma_memory_bytes(const LpmaHandle *h, uint64_t *bytes) {
         b += 18 * ns + nseg * (4 + 16 + 7 * 4) + bitmap_words(h->c.Hc) * 4;
     }
     b += 4ull * h->V + h->bcap * 64ull + h->view_cap * 9ull + h->exp_cap * 9ull + h->stage_cap * 34ull;
-    if (h->bfs_a) b += 8ull * h->V;
+    b += h->bfs_cap * 16ull;
     if (h->pr_deg) b += 20ull * h->V;
     b += h->q_cap * 8ull;
     *bytes = b;

@@ -160,11 +160,15 @@ void launch_nbr_fill(const uint32_t *srcs, const uint64_t *windows, uint32_t n, 
                      cudaStream_t s);
 void launch_edge_query(const uint64_t *q, uint32_t n, uint32_t window, Geo g, const ulonglong2 *fl,
                        const uint32_t *sent, uint32_t V, uint32_t *res, cudaStream_t s);
-void launch_bfs_init(const uint32_t *sources, uint32_t n, uint32_t V, int32_t *dist, uint32_t *frontier,
-                     uint32_t *count, cudaStream_t s);
-void launch_bfs_expand(const uint32_t *frontier, const uint32_t *nf, uint32_t nf_host, int32_t level, Geo g,
-                       const uint8_t *cnt, const uint32_t *sent, int32_t *dist, uint32_t *next, uint32_t *next_count,
-                       cudaStream_t s);
+// BFS frontiers: lists of slot ranges (linear slots [x, y) of a few
+// segments), at most bfs_items_for(V, H) of them; n_items / n_found are
+// device counters of the list's ranges and of the vertices found
+uint32_t bfs_items_for(uint32_t V, uint32_t H);
+void launch_bfs_init(const uint32_t *sources, uint32_t n, uint32_t V, Geo g, const uint32_t *sent, int32_t *dist,
+                     uint2 *items, uint32_t cap, uint32_t *n_items, uint32_t *n_found, cudaStream_t s);
+void launch_bfs_expand(const uint2 *items, const uint32_t *n_items, int32_t level, Geo g, const uint8_t *cnt,
+                       const uint32_t *sent, int32_t *dist, uint2 *next, uint32_t cap, uint32_t *n_next,
+                       uint32_t *n_found, cudaStream_t s);
 void launch_outdeg(Geo g, const uint8_t *cnt, uint32_t *deg, cudaStream_t s);
 void launch_fill_f64(double *p, uint64_t n, double x, cudaStream_t s);
 void launch_pr_iteration(Geo g, const uint8_t *cnt, const uint32_t *deg, uint32_t V, double alpha, double *rank,

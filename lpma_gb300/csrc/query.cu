@@ -224,47 +224,114 @@ __global__ void __launch_bounds__(TPB) k_edge_query(const uint64_t *__restrict__
 }
 
 // ---------------------------------------------------------------- BFS
+// A frontier is a list of slot ranges of at most BFS_SEGS segments each (a
+// vertex of many edges makes several), so the work of a level spreads over
+// the grid whatever the degrees are: one 8-lane group expands a range.  A
+// vertex found at this level gets dist = level + 1 and its ranges join the
+// next frontier; a warp queues what it finds and places 32 vertices with one
+// atomic.
+//
+// With a warp per frontier vertex the hubs of an R-MAT graph were walked by
+// one warp each: a 2-hop BFS from 1,024 seeds of a scale-20 graph (16.8M
+// edges) took 1,697 us of expansion, a full one 3,376; now 128 and 362 (280
+// and 524 with an atomic per find round: a million on one address).  Ranges
+// of 1, 2, 4 and 8 segments measured within 5%; 4 keeps the lists short.
+// Bound by the random reads of dist (one a stored edge, out of L2).
+constexpr uint32_t BFS_SEGS = 4;
+
+// the ranges of the vertices d of the lanes with `add` set (whole warps)
+__device__ inline void bfs_append(bool add, uint32_t d, Geo g, const uint32_t *__restrict__ sent, uint2 *items,
+                                  uint32_t cap, uint32_t *n_items) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint64_t p0 = 0, p1 = 0;
+    if (add) vertex_range(sent, d, g.H, p0, p1);
+    const uint32_t k = p1 > p0 ? (uint32_t)(((p1 - 1) >> 5) - (p0 >> 5)) / BFS_SEGS + 1 : 0u;
+    uint32_t incl = k;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
+    if (!tot) return;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(n_items, tot);
+    at = __shfl_sync(0xffffffffu, at, 0) + incl - k;
+    uint64_t a = p0;
+    for (uint32_t i = 0; i < k; i++) {
+        const uint64_t e = umin64(p1, ((a >> 5) + BFS_SEGS) << 5);
+        if (at + i < cap) items[at + i] = make_uint2((uint32_t)a, (uint32_t)e);
+        a = e;
+    }
+}
+
 __global__ void __launch_bounds__(TPB) k_bfs_init(int32_t *dist, uint32_t V) {
     for (uint64_t v = blockIdx.x * (uint64_t)TPB + threadIdx.x; v < V; v += gridDim.x * (uint64_t)TPB)
         dist[v] = INT_MAX;
 }
 
-__global__ void __launch_bounds__(TPB) k_bfs_seed(const uint32_t *__restrict__ sources, uint32_t n, uint32_t V,
-                                                  int32_t *dist, uint32_t *frontier, uint32_t *count) {
-    for (uint64_t i = blockIdx.x * (uint64_t)TPB + threadIdx.x; i < n; i += gridDim.x * (uint64_t)TPB) {
-        const uint32_t s = sources[i];
-        if (s < V && atomicCAS(&dist[s], INT_MAX, 0) == INT_MAX) frontier[atomicAdd(count, 1u)] = s;
+__global__ void __launch_bounds__(TPB) k_bfs_seed(const uint32_t *__restrict__ sources, uint32_t n, uint32_t V, Geo g,
+                                                  const uint32_t *__restrict__ sent, int32_t *dist, uint2 *items,
+                                                  uint32_t cap, uint32_t *n_items, uint32_t *n_found) {
+    for (uint64_t i0 = blockIdx.x * (uint64_t)TPB; i0 < n; i0 += gridDim.x * (uint64_t)TPB) {
+        const uint64_t i = i0 + threadIdx.x;
+        const uint32_t s = i < n ? sources[i] : V;
+        const bool add = s < V && atomicCAS(&dist[s], INT_MAX, 0) == INT_MAX;
+        const uint32_t c = __popc(__ballot_sync(0xffffffffu, add));
+        if (c && (threadIdx.x & 31) == 0) atomicAdd(n_found, c);
+        bfs_append(add, s, g, sent, items, cap, n_items);
     }
 }
 
-// one warp per frontier vertex; a neighbour first reached at this level gets
-// dist = level + 1 and joins the next frontier
-__global__ void __launch_bounds__(TPB) k_bfs_expand(const uint32_t *__restrict__ frontier,
-                                                    const uint32_t *__restrict__ nf_p, int32_t level, Geo g,
-                                                    const uint8_t *__restrict__ cnt,
-                                                    const uint32_t *__restrict__ sent, int32_t *dist, uint32_t *next,
-                                                    uint32_t *next_count) {
-    const int lane = threadIdx.x & 31, gl = lane & 7, grp = lane >> 3;
-    const uint32_t nf = *nf_p;
-    for (uint64_t i = (blockIdx.x * (uint64_t)TPB + threadIdx.x) >> 5; i < nf; i += (gridDim.x * (uint64_t)TPB) >> 5) {
-        const uint32_t u = frontier[i];
-        uint64_t p0, p1;
-        vertex_range(sent, u, g.H, p0, p1);
-        if (p1 <= p0) continue;
-        const uint64_t S0 = p0 >> 5, S1 = (p1 - 1) >> 5;
-        for (uint64_t s = S0 + grp; s <= S1; s += 4) {
+__global__ void __launch_bounds__(TPB) k_bfs_expand(const uint2 *__restrict__ items, const uint32_t *__restrict__ n_p,
+                                                    int32_t level, Geo g, const uint8_t *__restrict__ cnt,
+                                                    const uint32_t *__restrict__ sent, int32_t *dist, uint2 *next,
+                                                    uint32_t cap, uint32_t *n_next, uint32_t *n_found) {
+    // vertices found by a warp wait here until they fill it once
+    __shared__ uint32_t queue[TPB / 32][160];
+    uint32_t *Q = queue[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, gl = lane & 7;
+    const uint32_t n = min(*n_p, cap), stride = gridDim.x * (TPB / 8), lt = lanemask_lt();
+    uint32_t found = 0, nq = 0;
+    for (uint32_t i0 = (blockIdx.x * TPB + threadIdx.x) / 32 * 4; i0 < n; i0 += stride) {  // uniform over the warp
+        const uint32_t i = i0 + (lane >> 3);
+        const uint2 it = i < n ? items[i] : make_uint2(0u, 0u);
+        const uint32_t s0 = it.x >> 5, ns = it.y > it.x ? ((it.y - 1) >> 5) - s0 + 1 : 0u;
+        const uint32_t nmax = __reduce_max_sync(0xffffffffu, ns);
+        for (uint32_t r = 0; r < nmax; r++) {
             uint64_t k[4];
             uint8_t v[4];
-            const uint32_t m = load_seg_part(g, cnt, s, p0, p1, gl, k, v);
+            uint32_t m = 0;
+            if (r < ns) m = load_seg_part(g, cnt, s0 + r, it.x, it.y, gl, k, v);
+            uint32_t d[4];
+            // most neighbours are known already: a plain read comes before the
+            // compare-and-swap (a distance is written once)
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                if ((m >> q) & 1u) {
-                    const uint32_t d = (uint32_t)((k[q] & DST_MASK) >> DST_SHIFT);
-                    if (atomicCAS(&dist[d], INT_MAX, level + 1) == INT_MAX) next[atomicAdd(next_count, 1u)] = d;
-                }
+                d[q] = (uint32_t)((k[q] & DST_MASK) >> DST_SHIFT);
+                if (((m >> q) & 1u) && dist[d[q]] != INT_MAX) m &= ~(1u << q);
             }
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (((m >> q) & 1u) && atomicCAS(&dist[d[q]], INT_MAX, level + 1) != INT_MAX) m &= ~(1u << q);
+            found += __popc(m);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const uint32_t bal = __ballot_sync(0xffffffffu, (m >> q) & 1u);
+                if ((m >> q) & 1u) Q[nq + __popc(bal & lt)] = d[q];
+                nq += __popc(bal);
+            }
+            __syncwarp();
+            while (nq >= 32) {
+                nq -= 32;
+                bfs_append(true, Q[nq + lane], g, sent, next, cap, n_next);
+            }
+            __syncwarp();
         }
     }
+    bfs_append((uint32_t)lane < nq, (uint32_t)lane < nq ? Q[lane] : 0u, g, sent, next, cap, n_next);
+    found = __reduce_add_sync(0xffffffffu, found);
+    if (lane == 0 && found) atomicAdd(n_found, found);
 }
 
 // ---------------------------------------------------------------- PageRank
@@ -382,20 +449,24 @@ void launch_edge_query(const uint64_t *q, uint32_t n, uint32_t window, Geo g, co
     note_launch();
 }
 
-void launch_bfs_init(const uint32_t *sources, uint32_t n, uint32_t V, int32_t *dist, uint32_t *frontier,
-                     uint32_t *count, cudaStream_t s) {
+void launch_bfs_init(const uint32_t *sources, uint32_t n, uint32_t V, Geo g, const uint32_t *sent, int32_t *dist,
+                     uint2 *items, uint32_t cap, uint32_t *n_items, uint32_t *n_found, cudaStream_t s) {
     ProfScope ps_("bfs_init", s);
     k_bfs_init<<<grid_for(V, TPB, 152 * 16), TPB, 0, s>>>(dist, V);
-    k_bfs_seed<<<grid_for(n, TPB, 152 * 16), TPB, 0, s>>>(sources, n, V, dist, frontier, count);
+    k_bfs_seed<<<grid_for(n, TPB, 152 * 16), TPB, 0, s>>>(sources, n, V, g, sent, dist, items, cap, n_items, n_found);
     note_launch(2);
 }
 
-void launch_bfs_expand(const uint32_t *frontier, const uint32_t *nf, uint32_t nf_host, int32_t level, Geo g,
-                       const uint8_t *cnt, const uint32_t *sent, int32_t *dist, uint32_t *next, uint32_t *next_count,
-                       cudaStream_t s) {
+uint32_t bfs_items_for(uint32_t V, uint32_t H) { return (uint32_t)(V + (nseg_of(H) + V) / BFS_SEGS + 1); }
+
+void launch_bfs_expand(const uint2 *items, const uint32_t *n_items, int32_t level, Geo g, const uint8_t *cnt,
+                       const uint32_t *sent, int32_t *dist, uint2 *next, uint32_t cap, uint32_t *n_next,
+                       uint32_t *n_found, cudaStream_t s) {
     ProfScope ps_("bfs_expand", s);
-    k_bfs_expand<<<grid_for(nf_host, TPB / 32, 152 * 16), TPB, 0, s>>>(frontier, nf, level, g, cnt, sent, dist, next,
-                                                                       next_count);
+    // the list's length is known on the device only: a resident grid that
+    // loops (8 CTAs a SM), smaller for a graph that cannot fill it
+    k_bfs_expand<<<grid_for(cap, TPB / 8, 152 * 8), TPB, 0, s>>>(items, n_items, level, g, cnt, sent, dist, next, cap,
+                                                                 n_next, n_found);
     note_launch();
 }
 
