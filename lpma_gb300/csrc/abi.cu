@@ -134,7 +134,7 @@ struct LpmaHandle {
     uint64_t graph_clock = 0;
     bool host_staged = false;    // h2d already holds the staged input bytes
     // read paths (neighbour query, BFS, PageRank)
-    uint32_t *q_cnt = nullptr, *q_tmp = nullptr;
+    NbrScratch q{};
     size_t q_cap = 0;
     uint2 *bfs_a = nullptr, *bfs_b = nullptr;  // frontier lists
     uint32_t *bfs_cnt = nullptr;               // BFS_WORDS counters
@@ -1209,7 +1209,8 @@ lpma_status_t lpma_destroy(LpmaHandle *h) {
     if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
     dfree_async(h->row_offset), dfree_async(h->col_index), dfree_async(h->view_vals), dfree_async(h->exp_keys),
         dfree_async(h->exp_vals);
-    dfree_async(h->q_cnt), dfree_async(h->q_tmp), dfree_async(h->bfs_a), dfree_async(h->bfs_b),
+    dfree_async(h->q.rounds), dfree_async(h->q.at), dfree_async(h->q.base), dfree_async(h->q.done), dfree_async(h->q.tmp);
+    dfree_async(h->bfs_a), dfree_async(h->bfs_b),
         dfree_async(h->bfs_cnt);
     dfree_async(h->pr_deg), dfree_async(h->pr_contrib), dfree_async(h->pr_acc), dfree_async(h->pr_dangling);
     if (h->done_ev) cudaEventDestroy(h->done_ev);
@@ -1532,17 +1533,19 @@ lpma_status_t lpma_query_neighbors(LpmaHandle *h, const uint32_t *d_srcs, const 
     cudaStream_t s = (cudaStream_t)stream;
     if (!h->pin_word) CK(pinned_alloc(&h->pin_word, PIN_WORDS * sizeof(uint32_t)));
     if (n > h->q_cap) {
-        dfree(h->q_cnt), dfree(h->q_tmp);
+        dfree(h->q.rounds), dfree(h->q.at), dfree(h->q.tmp);
         h->q_cap = 0;
         const size_t c = std::max<size_t>(n, 1024);
-        CK(dalloc(&h->q_cnt, c));
-        CK(dalloc(&h->q_tmp, scan_tmp_words((uint32_t)c) + 64));
+        CK(dalloc(&h->q.rounds, c + 1));
+        CK(dalloc(&h->q.at, c));
+        CK(dalloc(&h->q.tmp, scan_tmp_words((uint32_t)c) + 64));
+        if (!h->q.base) CK(dalloc(&h->q.base, nbr_base_words()));
+        if (!h->q.done) CK(dalloc(&h->q.done, 1));
         h->q_cap = c;
     }
     Geo g{h->c.keys, h->c.vals, h->H};
     if (n) {
-        launch_nbr_count(d_srcs, d_windows, (uint32_t)n, g, h->c.cnt, h->sent, h->V, h->q_cnt, s);
-        CK(scan_u32(h->q_cnt, d_offsets, (uint32_t)n, d_offsets + n, h->q_tmp, s));
+        CK(launch_nbr_count(d_srcs, d_windows, (uint32_t)n, g, h->c.cnt, h->sent, h->V, h->q, d_offsets, s));
     } else {
         CK(cudaMemsetAsync(d_offsets, 0, sizeof(uint32_t), s));
     }
@@ -1551,7 +1554,7 @@ lpma_status_t lpma_query_neighbors(LpmaHandle *h, const uint32_t *d_srcs, const 
     *total = h->pin_word[0];
     if (!d_nbrs || !n) return LPMA_OK;
     if (*total > cap) return LPMA_ERR_BUFFER_TOO_SMALL;
-    launch_nbr_fill(d_srcs, d_windows, (uint32_t)n, g, h->c.cnt, h->sent, h->V, d_offsets, d_nbrs, d_vals, s);
+    launch_nbr_fill(d_srcs, d_windows, (uint32_t)n, g, h->c.cnt, h->sent, h->V, h->q, d_nbrs, d_vals, s);
     CK(cudaGetLastError());
     mark_done(h, s);
     return LPMA_OK;
@@ -1690,7 +1693,7 @@ lpma_status_t lpma_memory_bytes(const LpmaHandle *h, uint64_t *bytes) {
     b += 4ull * h->V + h->bcap * 64ull + h->view_cap * 9ull + h->exp_cap * 9ull + h->stage_cap * 34ull;
     b += h->bfs_cap * 16ull;
     if (h->pr_deg) b += 20ull * h->V;
-    b += h->q_cap * 8ull;
+    b += h->q_cap * 12ull;
     *bytes = b;
     return LPMA_OK;
 }

@@ -153,10 +153,21 @@ void launch_scatter_flags(const uint64_t *keys, const uint32_t *pos, const uint3
 
 
 // ---- read paths over the PMA (query.cu)
-void launch_nbr_count(const uint32_t *srcs, const uint64_t *windows, uint32_t n, Geo g, const uint8_t *cnt,
-                      const uint32_t *sent, uint32_t V, uint32_t *qcnt, cudaStream_t s);
+// Neighbour lists of n queries: the count writes offsets[0 .. n] and the
+// scratch that the fill of the same call reads.
+struct NbrScratch {
+    uint32_t *rounds;  // n + 1: each query's first round
+    uint2 *at;         // n: the share a query starts in, the share's neighbours before it
+    uint32_t *base;    // nbr_base_words(): where each share's neighbours start
+    uint32_t *done;    // one word: CTAs of the count that finished
+    uint32_t *tmp;     // scan_tmp_words(n)
+};
+size_t nbr_base_words();
+cudaError_t launch_nbr_count(const uint32_t *srcs, const uint64_t *windows, uint32_t n, Geo g, const uint8_t *cnt,
+                             const uint32_t *sent, uint32_t V, const NbrScratch &q, uint32_t *offsets,
+                             cudaStream_t s);
 void launch_nbr_fill(const uint32_t *srcs, const uint64_t *windows, uint32_t n, Geo g, const uint8_t *cnt,
-                     const uint32_t *sent, uint32_t V, const uint32_t *offsets, uint32_t *nbrs, uint8_t *vals,
+                     const uint32_t *sent, uint32_t V, const NbrScratch &q, uint32_t *nbrs, uint8_t *vals,
                      cudaStream_t s);
 void launch_edge_query(const uint64_t *q, uint32_t n, uint32_t window, Geo g, const ulonglong2 *fl,
                        const uint32_t *sent, uint32_t V, uint32_t *res, cudaStream_t s);

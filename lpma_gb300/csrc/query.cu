@@ -60,84 +60,219 @@ __device__ inline bool in_window(uint64_t key, uint32_t lb, uint32_t ub) {
 // ---------------------------------------------------------------- neighbour lists
 // query_rpma (rpma.cuh:1827-2036): for query i, the neighbours of srcs[i]
 // whose timestamp lies in [windows[i] >> 32, windows[i] & 0xFFFFFFFF], in
-// key order.  One warp per query, four segments per round (one per 8-lane
-// group).  Pass 1 counts, pass 2 writes at offsets[i].
+// key order.
+//
+// The queries' rounds (4 segments, one per 8-lane group of a warp; at least
+// one round a query) are laid end to end and cut into equal shares, one a
+// warp, so a hub's list is read by many warps.  The lists too lie end to end
+// in that order: a share's neighbours start where those of the shares
+// before it end.  Pass 1 counts each share (and, for each query that starts
+// in it, the share's neighbours before that query); its last CTA sums the
+// shares; pass 2 writes.  A warp per query walked the hubs serially: 4,096
+// lists of a scale-20 graph, 8 hubs among them, took 240 us a count and 335 a
+// fill, now 24 and 11 (and 12 to weigh the queries).
+//
+// A query counts as nbr_cap(n) rounds at most, so that the rounds of all n
+// stay below 2^31; one of more is cut into that many equal parts.
+constexpr uint32_t NBR_CTAS = 152 * 4, NBR_SHARES = NBR_CTAS * (TPB / 32);
+constexpr uint32_t NBR_ONE_CTA = 8192;  // up to here one CTA weighs the queries, and one places the lists
+
+__host__ __device__ inline uint32_t nbr_cap(uint32_t n) { return ((1u << 31) - 1) / n; }
+
+__device__ __forceinline__ uint32_t nbr_rounds(uint32_t src, uint32_t n, uint32_t V, Geo g, const uint32_t *sent) {
+    if (src >= V) return 1;
+    uint64_t p0, p1;
+    vertex_range(sent, src, g.H, p0, p1);
+    return p1 > p0 ? min((uint32_t)(((p1 - 1) >> 5) - (p0 >> 5)) / 4 + 1, nbr_cap(n)) : 1u;
+}
+
+// rounds of every query (scanned afterwards)
+__global__ void __launch_bounds__(TPB) k_nbr_weigh(const uint32_t *__restrict__ srcs, uint32_t n, Geo g,
+                                                   const uint32_t *__restrict__ sent, uint32_t V, uint32_t *w) {
+    for (uint32_t i = blockIdx.x * TPB + threadIdx.x; i < n; i += gridDim.x * TPB)
+        w[i] = nbr_rounds(srcs[i], n, V, g, sent);
+}
+
+// the same and the exclusive scan for up to NBR_ONE_CTA queries, in one CTA
+__global__ void __launch_bounds__(1024) k_nbr_weigh_scan(const uint32_t *__restrict__ srcs, uint32_t n, Geo g,
+                                                         const uint32_t *__restrict__ sent, uint32_t V,
+                                                         uint32_t *P) {
+    constexpr uint32_t PER = NBR_ONE_CTA / 1024;
+    __shared__ uint32_t ws[32];
+    const uint32_t lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const uint32_t per = (n + 1023) / 1024, beg = threadIdx.x * per;
+    uint32_t x[PER], sum = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < PER; q++) {
+        x[q] = q < per && beg + q < n ? nbr_rounds(srcs[beg + q], n, V, g, sent) : 0u;
+        sum += x[q];
+    }
+    uint32_t v = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= (uint32_t)o) v += y;
+    }
+    if (lane == 31) ws[wp] = v;
+    __syncthreads();
+    uint32_t off = v - sum, tot = 0;
+    for (uint32_t k = 0; k < 32; k++) {
+        const uint32_t y = ws[k];
+        off += k < wp ? y : 0u;
+        tot += y;
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < PER; q++) {
+        if (q < per && beg + q < n) P[beg + q] = off;
+        off += x[q];
+    }
+    if (threadIdx.x == 0) P[n] = tot;
+}
+
+// Walks the rounds of share w: f(i, first, s0, s1, p0, p1, window) for each
+// query i in it (whole warps), first when the share holds its first round;
+// segments [s0, s1) of it, none for a query without slots.
+template <typename F>
+__device__ __forceinline__ void nbr_walk(uint32_t w, const uint32_t *__restrict__ srcs,
+                                         const uint64_t *__restrict__ windows, uint32_t n, Geo g,
+                                         const uint32_t *__restrict__ sent, uint32_t V,
+                                         const uint32_t *__restrict__ P, F f) {
+    const uint64_t T = P[n];
+    const uint32_t u0 = (uint32_t)(T * w / NBR_SHARES), u1 = (uint32_t)(T * (w + 1) / NBR_SHARES);
+    if (u0 >= u1) return;
+    uint32_t i = forest_job_of(P, n, u0);
+    for (uint32_t u = u0; u < u1; i++) {
+        const uint32_t qs = P[i], qe = P[i + 1];
+        const uint32_t a = u - qs, b = min(u1, qe) - qs;  // rounds [a, b) of query i
+        const uint32_t src = srcs[i];
+        const uint64_t win = windows[i];
+        uint64_t p0 = 0, p1 = 0;
+        if (src < V) vertex_range(sent, src, g.H, p0, p1);
+        uint32_t s0 = 0, s1 = 0;
+        if (p1 > p0) {
+            const uint32_t S0 = (uint32_t)(p0 >> 5), ns = (uint32_t)((p1 - 1) >> 5) + 1 - S0;
+            const uint32_t per = 4 * (((ns + 3) / 4 + qe - qs - 1) / (qe - qs));  // segments a round stands for
+            s0 = S0 + (uint32_t)umin64(ns, (uint64_t)a * per);
+            s1 = S0 + (uint32_t)umin64(ns, (uint64_t)b * per);
+        }
+        f(i, a == 0, s0, s1, p0, p1, win);
+        u = qs + b;
+    }
+}
+
 __global__ void __launch_bounds__(TPB) k_nbr_count(const uint32_t *__restrict__ srcs,
                                                    const uint64_t *__restrict__ windows, uint32_t n, Geo g,
                                                    const uint8_t *__restrict__ cnt, const uint32_t *__restrict__ sent,
-                                                   uint32_t V, uint32_t *qcnt) {
+                                                   uint32_t V, const uint32_t *__restrict__ P, uint32_t *done, uint2 *at,
+                                                   uint32_t *base, uint32_t *offsets) {
     const int lane = threadIdx.x & 31, gl = lane & 7, grp = lane >> 3;
-    for (uint64_t i = (blockIdx.x * (uint64_t)TPB + threadIdx.x) >> 5; i < n; i += (gridDim.x * (uint64_t)TPB) >> 5) {
-        const uint32_t src = srcs[i];
-        uint32_t total = 0;
-        if (src < V) {
-            const uint64_t w = windows[i];
-            const uint32_t lb = (uint32_t)(w >> 32), ub = (uint32_t)w;
-            uint64_t p0, p1;
-            vertex_range(sent, src, g.H, p0, p1);
-            if (p1 > p0) {
-                const uint64_t S0 = p0 >> 5, S1 = (p1 - 1) >> 5;
-                for (uint64_t s = S0 + grp; s <= S1; s += 4) {
-                    uint64_t k[4];
-                    uint8_t v[4];
-                    const uint32_t m = load_seg_part(g, cnt, s, p0, p1, gl, k, v);
+    const uint32_t w = (blockIdx.x * TPB + threadIdx.x) >> 5;
+    uint32_t run = 0;  // the share's neighbours so far
+    nbr_walk(w, srcs, windows, n, g, sent, V, P,
+             [&](uint32_t i, bool first, uint32_t s0, uint32_t s1, uint64_t p0, uint64_t p1, uint64_t win) {
+                 if (first && lane == 0) at[i] = make_uint2(w, run);
+                 const uint32_t lb = (uint32_t)(win >> 32), ub = (uint32_t)win;
+                 uint32_t c = 0;
+                 for (uint32_t s = s0 + grp; s < s1; s += 4) {
+                     uint64_t k[4];
+                     uint8_t v[4];
+                     const uint32_t m = load_seg_part(g, cnt, s, p0, p1, gl, k, v);
 #pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        if (((m >> q) & 1u) && in_window(k[q], lb, ub)) total++;
-                }
-            }
-        }
+                     for (int q = 0; q < 4; q++)
+                         if (((m >> q) & 1u) && in_window(k[q], lb, ub)) c++;
+                 }
+                 run += __reduce_add_sync(0xffffffffu, c);
+             });
+    if (lane == 0) base[w] = run;
+    // the last CTA to finish turns the shares' counts into their starts
+    __shared__ uint32_t last;
+    __shared__ uint32_t ws[TPB / 32];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1 ? 1u : 0u;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    constexpr uint32_t PER = NBR_SHARES / TPB;
+    static_assert(NBR_SHARES % TPB == 0, "equal runs of shares a thread");
+    uint32_t x[PER], sum = 0;
 #pragma unroll
-        for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-        if (lane == 0) qcnt[i] = total;
+    for (uint32_t q = 0; q < PER; q++) sum += x[q] = __ldcg(base + threadIdx.x * PER + q);
+    uint32_t v = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
     }
+    if (lane == 31) ws[threadIdx.x >> 5] = v;
+    __syncthreads();
+    uint32_t off = v - sum, tot = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < TPB / 32; k++) {
+        const uint32_t y = ws[k];
+        off += k < (threadIdx.x >> 5) ? y : 0u;
+        tot += y;
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < PER; q++) {
+        base[threadIdx.x * PER + q] = off;
+        off += x[q];
+    }
+    if (threadIdx.x == 0) offsets[n] = tot;
+    if (n > NBR_ONE_CTA) return;  // k_nbr_offsets places the lists
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n; i += TPB) {
+        const uint32_t sw = __ldcg(&at[i].x), sr = __ldcg(&at[i].y);
+        offsets[i] = __ldcg(base + sw) + sr;
+    }
+}
+
+__global__ void __launch_bounds__(TPB) k_nbr_offsets(uint32_t n, const uint2 *__restrict__ at,
+                                                     const uint32_t *__restrict__ base, uint32_t *offsets) {
+    const uint32_t i = blockIdx.x * TPB + threadIdx.x;
+    if (i < n) offsets[i] = base[at[i].x] + at[i].y;
 }
 
 __global__ void __launch_bounds__(TPB) k_nbr_fill(const uint32_t *__restrict__ srcs,
                                                   const uint64_t *__restrict__ windows, uint32_t n, Geo g,
                                                   const uint8_t *__restrict__ cnt, const uint32_t *__restrict__ sent,
-                                                  uint32_t V, const uint32_t *__restrict__ offsets, uint32_t *nbrs,
-                                                  uint8_t *vals) {
+                                                  uint32_t V, const uint32_t *__restrict__ P,
+                                                  const uint32_t *__restrict__ base, uint32_t *nbrs, uint8_t *vals) {
     const int lane = threadIdx.x & 31, gl = lane & 7, grp = lane >> 3;
-    for (uint64_t i = (blockIdx.x * (uint64_t)TPB + threadIdx.x) >> 5; i < n; i += (gridDim.x * (uint64_t)TPB) >> 5) {
-        const uint32_t src = srcs[i];
-        if (src >= V) continue;  // warp-uniform
-        const uint64_t w = windows[i];
-        const uint32_t lb = (uint32_t)(w >> 32), ub = (uint32_t)w;
-        uint64_t p0, p1;
-        vertex_range(sent, src, g.H, p0, p1);
-        if (p1 <= p0) continue;
-        const uint64_t S0 = p0 >> 5, S1 = (p1 - 1) >> 5;
-        uint32_t out = offsets[i];
-        for (uint64_t s0 = S0; s0 <= S1; s0 += 4) {
-            const uint64_t s = s0 + grp;
-            uint64_t k[4];
-            uint8_t v[4];
-            uint32_t m = 0;
-            if (s <= S1) m = load_seg_part(g, cnt, s, p0, p1, gl, k, v);
+    const uint32_t w = (blockIdx.x * TPB + threadIdx.x) >> 5;
+    uint32_t out = base[w];
+    nbr_walk(w, srcs, windows, n, g, sent, V, P,
+             [&](uint32_t, bool, uint32_t s0, uint32_t s1, uint64_t p0, uint64_t p1, uint64_t win) {
+                 const uint32_t lb = (uint32_t)(win >> 32), ub = (uint32_t)win;
+                 for (uint32_t sr = s0; sr < s1; sr += 4) {
+                     const uint32_t s = sr + grp;
+                     uint64_t k[4];
+                     uint8_t v[4];
+                     uint32_t m = 0;
+                     if (s < s1) m = load_seg_part(g, cnt, s, p0, p1, gl, k, v);
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (((m >> q) & 1u) && !in_window(k[q], lb, ub)) m &= ~(1u << q);
-            // warp-wide exclusive prefix in (group, lane, slot) order = key order
-            const uint32_t c = __popc(m);
-            uint32_t incl = c;
+                     for (int q = 0; q < 4; q++)
+                         if (((m >> q) & 1u) && !in_window(k[q], lb, ub)) m &= ~(1u << q);
+                     // warp-wide exclusive prefix in (group, lane, slot) order = key order
+                     const uint32_t c = __popc(m);
+                     uint32_t incl = c;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            uint32_t pos = out + incl - c;
+                     for (int o = 1; o < 32; o <<= 1) {
+                         const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                         if (lane >= o) incl += y;
+                     }
+                     uint32_t pos = out + incl - c;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                if ((m >> q) & 1u) {
-                    nbrs[pos] = (uint32_t)((k[q] & DST_MASK) >> DST_SHIFT);
-                    vals[pos] = v[q];
-                    pos++;
-                }
-            }
-            out += __shfl_sync(0xffffffffu, incl, 31);
-        }
-    }
+                     for (int q = 0; q < 4; q++) {
+                         if ((m >> q) & 1u) {
+                             nbrs[pos] = (uint32_t)((k[q] & DST_MASK) >> DST_SHIFT);
+                             vals[pos] = v[q];
+                             pos++;
+                         }
+                     }
+                     out += __shfl_sync(0xffffffffu, incl, 31);
+                 }
+             });
 }
 
 // ---------------------------------------------------------------- edge queries
@@ -426,21 +561,40 @@ inline uint32_t grid_for(uint64_t n, uint32_t per_block, uint32_t cap = 152 * 16
 
 }  // namespace
 
-void launch_nbr_count(const uint32_t *srcs, const uint64_t *windows, uint32_t n, Geo g, const uint8_t *cnt,
-                      const uint32_t *sent, uint32_t V, uint32_t *qcnt, cudaStream_t s) {
+cudaError_t launch_nbr_count(const uint32_t *srcs, const uint64_t *windows, uint32_t n, Geo g, const uint8_t *cnt,
+                             const uint32_t *sent, uint32_t V, const NbrScratch &q, uint32_t *offsets,
+                             cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(q.done, 0, sizeof(uint32_t), s);
+    if (e != cudaSuccess) return e;
+    if (n <= NBR_ONE_CTA) {
+        ProfScope ps_("nbr_weigh", s);
+        k_nbr_weigh_scan<<<1, 1024, 0, s>>>(srcs, n, g, sent, V, q.rounds);
+        note_launch();
+    } else {
+        ProfScope ps_("nbr_weigh", s);
+        k_nbr_weigh<<<grid_for(n, TPB, 152 * 8), TPB, 0, s>>>(srcs, n, g, sent, V, q.rounds);
+        note_launch();
+        if ((e = scan_u32(q.rounds, q.rounds, n, q.rounds + n, q.tmp, s)) != cudaSuccess) return e;
+    }
     ProfScope ps_("nbr_count", s);
-    k_nbr_count<<<grid_for(n, TPB / 32, 152 * 16), TPB, 0, s>>>(srcs, windows, n, g, cnt, sent, V, qcnt);
+    k_nbr_count<<<NBR_CTAS, TPB, 0, s>>>(srcs, windows, n, g, cnt, sent, V, q.rounds, q.done, q.at, q.base, offsets);
     note_launch();
+    if (n > NBR_ONE_CTA) {
+        k_nbr_offsets<<<(n + TPB - 1) / TPB, TPB, 0, s>>>(n, q.at, q.base, offsets);
+        note_launch();
+    }
+    return cudaGetLastError();
 }
 
 void launch_nbr_fill(const uint32_t *srcs, const uint64_t *windows, uint32_t n, Geo g, const uint8_t *cnt,
-                     const uint32_t *sent, uint32_t V, const uint32_t *offsets, uint32_t *nbrs, uint8_t *vals,
+                     const uint32_t *sent, uint32_t V, const NbrScratch &q, uint32_t *nbrs, uint8_t *vals,
                      cudaStream_t s) {
     ProfScope ps_("nbr_fill", s);
-    k_nbr_fill<<<grid_for(n, TPB / 32, 152 * 16), TPB, 0, s>>>(srcs, windows, n, g, cnt, sent, V, offsets, nbrs,
-                                                                vals);
+    k_nbr_fill<<<NBR_CTAS, TPB, 0, s>>>(srcs, windows, n, g, cnt, sent, V, q.rounds, q.base, nbrs, vals);
     note_launch();
 }
+
+size_t nbr_base_words() { return NBR_SHARES; }
 
 void launch_edge_query(const uint64_t *q, uint32_t n, uint32_t window, Geo g, const ulonglong2 *fl,
                        const uint32_t *sent, uint32_t V, uint32_t *res, cudaStream_t s) {

@@ -1,7 +1,8 @@
 """Read paths whose work is split by segments, at the edges of the split:
 hubs whose slots fill a few segments more or less than one range of the BFS
 frontier (4 segments of 32 slots), vertices without edges, every source the
-same."""
+same; neighbour lists of one query, of many, at the size up to which one CTA
+places them, and of so many that a hub's rounds are capped."""
 import numpy as np
 import pytest
 
@@ -45,4 +46,65 @@ def test_bfs_hub_ranges(engine, oracle, deg):
         # a level counts when it had a frontier to expand
         most = int(seen.max()) + 1 if seen.size else 0
         assert levels == (min(most, depth) if depth else most), (deg, sources, depth, levels)
+    g.close()
+
+
+def _lists(k, v, srcs, wins, V):
+    """(offsets, neighbours, values), vectorised over the queries."""
+    src, dst = (k >> np.uint64(42)).astype(np.int64), (k >> np.uint64(20)) & np.uint64(0x3FFFFF)
+    t = (k & np.uint64(0xFFFFF)).astype(np.int64)
+    edge = dst != 0x3FFFFE
+    src, dst, t, v = src[edge], dst[edge], t[edge], v[edge]
+    start = np.searchsorted(src, np.arange(V + 1))
+    s = np.asarray(srcs, np.int64)
+    inside = s < V
+    a, b = np.where(inside, start[np.minimum(s, V - 1)], 0), np.where(inside, start[np.minimum(s, V - 1) + 1], 0)
+    row = np.repeat(np.arange(s.size), b - a)
+    at = np.arange(row.size) - np.repeat(np.cumsum(b - a) - (b - a), b - a) + np.repeat(a, b - a)
+    w = np.asarray(wins, np.uint64)
+    lb, ub = (w >> np.uint64(32)).astype(np.int64), (w & np.uint64(0xFFFFFFFF)).astype(np.int64)
+    ok = (t[at] >= lb[row]) & (t[at] <= ub[row])
+    offs = np.concatenate([[0], np.cumsum(np.bincount(row[ok], minlength=s.size))])
+    return offs, dst[at][ok].astype(np.int64), v[at][ok]
+
+
+def _check_lists(g, k, v, srcs, wins, V):
+    offs, nb, nv = g.query_neighbors(_u32(srcs), _dev(wins))
+    eo, en, ev = _lists(k, v, srcs, wins, V)
+    assert np.array_equal(offs.cpu().numpy().view(np.uint32).astype(np.int64), eo)
+    assert np.array_equal(nb.cpu().numpy().astype(np.int64), en)
+    assert np.array_equal(nv.cpu().numpy(), ev)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 1023, 1025, 4864, 8191, 8192, 8193, 30000])
+def test_neighbor_lists_of_n_queries(engine, n):
+    g, (k, v) = _hub_graph(engine, 2900)
+    rng = np.random.default_rng(n)
+    srcs = rng.integers(0, 3100, n)  # some beyond the last vertex
+    srcs[rng.random(n) < 0.02] = 5   # the hub, again and again
+    srcs[0] = 5
+    wins = np.full(n, 0xFFFFF, np.uint64)
+    wins[rng.random(n) < 0.2] = np.uint64(3 << 32 | 9)  # holds nothing
+    _check_lists(g, k, v, srcs, wins, 3000)
+    _check_lists(g, k, v, np.full(n, 2999), wins, 3000)  # empty lists only
+    g.close()
+
+
+def test_neighbor_lists_with_capped_rounds(engine):
+    """2^20 queries: a query counts as at most 2,047 rounds of 4 segments;
+    the hub's 400,000 neighbours take more."""
+    V, n = 1 << 19, 1 << 20
+    rng = np.random.default_rng(1)
+    t = np.zeros(400000, np.uint64)
+    t[::1000] = 7
+    keys = (np.uint64(11) << np.uint64(42)) | (rng.permutation(V - 20)[:400000].astype(np.uint64) << np.uint64(20)) | t
+    keys = np.concatenate([keys, (np.arange(100, dtype=np.uint64) << np.uint64(42)) | np.uint64(3 << 20)])
+    g = engine.Lpma(V)
+    g.update(ins=_dev(np.unique(keys)))
+    k, v = g.export_sorted()
+    srcs = rng.integers(0, V, n)
+    srcs[[0, 5, n // 2, n - 1]] = 11
+    wins = np.full(n, 0xFFFFF, np.uint64)
+    wins[[5, n - 1]] = np.uint64(7 << 32 | 7)
+    _check_lists(g, k, v, srcs, wins, V)
     g.close()
