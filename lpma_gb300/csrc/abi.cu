@@ -155,6 +155,16 @@ struct LpmaHandle {
 
 namespace {
 
+// When PageRank lays the edges out by destination first (query.cu).  The
+// layout costs a pushed iteration or two and its iterations are fewer
+// launches with a floor of 19 us, so it pays from three iterations and 3M
+// pushed edges on (us, push / pull: 16.8M edges 2 iterations 809 / 811, 3
+// 1,118 / 785, 20 6,375 / 2,933; 1M edges 3 193 / 161; 524K 4 148 / 169, 8
+// 271 / 251; 262K 20 513 / 492; 131K 20 426 / 489).
+bool pagerank_pulls(uint64_t edges, uint32_t iterations) {
+    return iterations >= 3 && edges >= (1u << 17) && edges * iterations >= (3u << 20);
+}
+
 // levels of a BFS launched before the host reads their counters back, the
 // counters of those levels (ranges and vertices of each frontier), and the
 // words of the read paths' pinned buffer
@@ -1634,9 +1644,35 @@ lpma_status_t lpma_pagerank(LpmaHandle *h, double alpha, uint32_t iterations, do
         CK(dalloc(&h->pr_deg, h->V));
         CK(dalloc(&h->pr_contrib, h->V));
         CK(dalloc(&h->pr_acc, h->V));
-        CK(dalloc(&h->pr_dangling, 1));
+        CK(dalloc(&h->pr_dangling, 3));
     }
     const Geo g{h->c.keys, h->c.vals, h->H};
+    if (pagerank_pulls(h->total - h->V, iterations)) {
+        // the edges by destination and the reciprocal degrees, for this call
+        PrLayout l;
+        const uint64_t words = pr_words(h->V, h->total - h->V, &l);
+        const size_t at = (words * 4 + 255) & ~size_t(255);
+        void *mem = nullptr;
+        const cudaError_t e = pool_alloc(&mem, at + sizeof(double) * h->V, s);
+        if (e == cudaSuccess) {
+            uint32_t *w = static_cast<uint32_t *>(mem);
+            double *inv = reinterpret_cast<double *>(static_cast<char *>(mem) + at);
+            const uint64_t nseg = nseg_of(h->H);
+            cudaError_t x = scan_u8_to_u32(h->c.cnt, h->c.segP, (uint32_t)nseg, h->c.segP + nseg, h->c.scan_tmp, s);
+            if (!x) x = launch_pr_layout(g, h->c.cnt, h->c.segP, h->sent, h->V, l, w, inv, h->pr_deg, s);
+            if (!x) x = cudaMemsetAsync(h->pr_dangling, 0, 3 * sizeof(double), s);
+            for (uint32_t it = 0; it <= iterations && !x; it++)
+                launch_pr_pull(it, l, w, h->V, alpha, inv, h->pr_deg, d_rank, h->pr_contrib, h->pr_acc, h->pr_dangling,
+                               s);
+            if (!x) x = cudaGetLastError();
+            const cudaError_t f = cudaFreeAsync(mem, s);
+            CK(x);
+            CK(f);
+            mark_done(h, s);
+            return LPMA_OK;
+        }
+        cudaGetLastError();  // no room for the edges: the push form below needs none
+    }
     CK(cudaMemsetAsync(h->pr_deg, 0, sizeof(uint32_t) * h->V, s));
     CK(cudaMemsetAsync(h->pr_acc, 0, sizeof(double) * h->V, s));
     launch_outdeg(g, h->c.cnt, h->pr_deg, s);

@@ -182,6 +182,19 @@ void launch_bfs_expand(const uint2 *items, const uint32_t *n_items, int32_t leve
                        uint32_t *n_found, cudaStream_t s);
 void launch_outdeg(Geo g, const uint8_t *cnt, uint32_t *deg, cudaStream_t s);
 void launch_fill_f64(double *p, uint64_t n, double x, cudaStream_t s);
+// The edges by destination for a PageRank of several iterations (`words`:
+// pr_words() 32-bit words, 16-byte aligned; P: exclusive prefix of the
+// segment counts), then iteration 0 (the start) and 1, 2, ... ; dangling
+// holds three sums, zero before iteration 0.
+struct PrLayout {
+    uint32_t nbins, max_chunks, cap;
+};
+size_t pr_words(uint32_t V, uint64_t edges, PrLayout *l);
+cudaError_t launch_pr_layout(Geo g, const uint8_t *cnt, const uint32_t *P, const uint32_t *sent, uint32_t V,
+                             const PrLayout &l, uint32_t *words, double *inv, uint32_t *deg, cudaStream_t s);
+void launch_pr_pull(uint32_t it, const PrLayout &l, const uint32_t *words, uint32_t V, double alpha, const double *inv,
+                    const uint32_t *deg, double *rank, double *contrib, double *acc, double *dangling,
+                    cudaStream_t s);
 void launch_pr_iteration(Geo g, const uint8_t *cnt, const uint32_t *deg, uint32_t V, double alpha, double *rank,
                          double *contrib, double *acc, double *dangling, cudaStream_t s);
 

@@ -550,6 +550,252 @@ __global__ void __launch_bounds__(TPB) k_pr_finish(double *rank, double *acc, ui
 
 __global__ void k_zero_f64(double *p) { *p = 0.0; }
 
+// PageRank of several iterations reads the edges by destination instead.
+// The edges are laid out once per call as 32-bit words src << 10 | (dst mod
+// 1024), grouped by dst / 1024 (a bin), each bin cut into chunks of up to
+// PR_CHUNK edges that are sorted by destination.  An iteration is then a sum
+// over runs of equal destinations: one CTA a chunk, 32 consecutive edges a
+// thread, a run inside a thread's edges stored once, one that crosses
+// threads added in shared memory; a chunk adds at most 1,024 sums to acc.
+//
+// The push form (k_pr_push) makes one f64 atomic an edge: 276-300 us an
+// iteration on a scale-20 graph (16.8M edges).  This form takes 124 after
+// 356 for the layout; bound by the random 8-byte reads of contrib (one a
+// stored edge, out of L2: 5.4 TB/s of 32-byte sectors).
+constexpr uint32_t PR_LOW = 10, PR_BIN = 1u << PR_LOW, PR_MAX_BINS = 4096, PR_CHUNK = 16384;
+constexpr uint32_t PR_SORT_TPB = 1024, PR_PULL_TPB = 512, PR_EPT = PR_CHUNK / PR_PULL_TPB;
+constexpr uint32_t PR_TILE_SEGS = 512;  // segments a CTA counts or places
+
+// the edges of segment s: f(src, dst) on each of the group's lanes
+template <typename F>
+__device__ __forceinline__ void seg_edges(Geo g, const uint8_t *__restrict__ cnt, uint64_t s, int gl, F f) {
+    uint64_t k[4];
+    uint8_t v[4];
+    const uint32_t m = load_seg_part(g, cnt, s, 0, ~0ull, gl, k, v);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (((m >> q) & 1u) && !is_sentinel(k[q]))
+            f((uint32_t)(k[q] >> SRC_SHIFT), (uint32_t)((k[q] & DST_MASK) >> DST_SHIFT));
+}
+
+__global__ void __launch_bounds__(TPB) k_pr_count(Geo g, const uint8_t *__restrict__ cnt, uint32_t nbins,
+                                                  uint32_t *bins) {
+    __shared__ uint32_t hist[PR_MAX_BINS];
+    for (uint32_t b = threadIdx.x; b < nbins; b += TPB) hist[b] = 0;
+    __syncthreads();
+    const uint64_t nseg = nseg_of(g.H), t0 = (uint64_t)blockIdx.x * PR_TILE_SEGS;
+    for (uint32_t r = threadIdx.x >> 3; r < PR_TILE_SEGS; r += TPB / 8)
+        if (t0 + r < nseg)
+            seg_edges(g, cnt, t0 + r, threadIdx.x & 7,
+                      [&](uint32_t, uint32_t dst) { atomicAdd(&hist[dst >> PR_LOW], 1u); });
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < nbins; b += TPB)
+        if (hist[b]) atomicAdd(&bins[b], hist[b]);
+}
+
+// one CTA: bins[b] (counts) -> where each bin starts (multiples of 4 words),
+// the cursors of the placing, and the chunks (first word, edges, bin, the
+// bin's chunks)
+__global__ void __launch_bounds__(1024) k_pr_table(uint32_t nbins, uint32_t *bins, uint4 *chunks,
+                                                   uint32_t *n_chunks) {
+    constexpr uint32_t PER = PR_MAX_BINS / 1024;
+    __shared__ uint64_t ws[32];
+    const uint32_t lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    uint32_t c[PER];
+    uint64_t sum = 0;  // words in the low half (below 2^32: at most 2^30 keys), chunks in the high
+#pragma unroll
+    for (uint32_t q = 0; q < PER; q++) {
+        const uint32_t b = threadIdx.x * PER + q;
+        c[q] = b < nbins ? bins[b] : 0u;
+        sum += (uint64_t)((c[q] + 3) & ~3u) | ((uint64_t)((c[q] + PR_CHUNK - 1) / PR_CHUNK) << 32);
+    }
+    uint64_t v = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= (uint32_t)o) v += y;
+    }
+    if (lane == 31) ws[wp] = v;
+    __syncthreads();
+    uint64_t off = v - sum, tot = 0;
+    for (uint32_t k = 0; k < 32; k++) {
+        off += k < wp ? ws[k] : 0u;
+        tot += ws[k];
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < PER; q++) {
+        const uint32_t b = threadIdx.x * PER + q;
+        if (b >= nbins) break;
+        const uint32_t nch = (c[q] + PR_CHUNK - 1) / PR_CHUNK;
+        bins[b] = (uint32_t)off;
+        for (uint32_t k = 0; k < nch; k++)
+            chunks[(uint32_t)(off >> 32) + k] =
+                make_uint4((uint32_t)off + k * PR_CHUNK, min(PR_CHUNK, c[q] - k * PR_CHUNK), b, nch);
+        off += (uint64_t)((c[q] + 3) & ~3u) | ((uint64_t)nch << 32);
+    }
+    if (threadIdx.x == 0) *n_chunks = (uint32_t)(tot >> 32);
+}
+
+// every edge to its bin: a CTA counts its tile's edges per bin, takes its
+// places in each bin with one atomic, and writes them
+__global__ void __launch_bounds__(TPB) k_pr_place(Geo g, const uint8_t *__restrict__ cnt, uint32_t nbins,
+                                                  uint32_t *cursor, uint32_t *edges, uint32_t cap) {
+    __shared__ uint32_t at[PR_MAX_BINS];
+    for (uint32_t b = threadIdx.x; b < nbins; b += TPB) at[b] = 0;
+    __syncthreads();
+    const uint64_t nseg = nseg_of(g.H), t0 = (uint64_t)blockIdx.x * PR_TILE_SEGS;
+    for (uint32_t r = threadIdx.x >> 3; r < PR_TILE_SEGS; r += TPB / 8)
+        if (t0 + r < nseg)
+            seg_edges(g, cnt, t0 + r, threadIdx.x & 7,
+                      [&](uint32_t, uint32_t dst) { atomicAdd(&at[dst >> PR_LOW], 1u); });
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < nbins; b += TPB)
+        if (at[b]) at[b] = atomicAdd(&cursor[b], at[b]);
+    __syncthreads();
+    for (uint32_t r = threadIdx.x >> 3; r < PR_TILE_SEGS; r += TPB / 8)
+        if (t0 + r < nseg)
+            seg_edges(g, cnt, t0 + r, threadIdx.x & 7, [&](uint32_t src, uint32_t dst) {
+                const uint32_t p = atomicAdd(&at[dst >> PR_LOW], 1u);
+                if (p < cap) edges[p] = (src << PR_LOW) | (dst & (PR_BIN - 1));
+            });
+}
+
+// each chunk sorted by destination, in place (a counting sort in shared memory)
+__global__ void __launch_bounds__(PR_SORT_TPB) k_pr_sort(const uint4 *__restrict__ chunks,
+                                                         const uint32_t *__restrict__ n_chunks, uint32_t *edges) {
+    extern __shared__ __align__(16) uint32_t sm[];
+    uint32_t *e = sm, *o = sm + PR_CHUNK, *at = sm + 2 * PR_CHUNK, *ws = at + PR_BIN;
+    static_assert(PR_SORT_TPB == PR_BIN, "a counter a thread");
+    if (blockIdx.x >= *n_chunks) return;
+    const uint4 c = chunks[blockIdx.x];
+    const uint32_t lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    at[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < c.y; i += PR_SORT_TPB) {
+        e[i] = edges[c.x + i];
+        atomicAdd(&at[e[i] & (PR_BIN - 1)], 1u);
+    }
+    __syncthreads();
+    const uint32_t x = at[threadIdx.x];
+    uint32_t v = x;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, k);
+        if (lane >= (uint32_t)k) v += y;
+    }
+    if (lane == 31) ws[wp] = v;
+    __syncthreads();
+    uint32_t off = v - x;
+    for (uint32_t k = 0; k < wp; k++) off += ws[k];
+    at[threadIdx.x] = off;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < c.y; i += PR_SORT_TPB) o[atomicAdd(&at[e[i] & (PR_BIN - 1)], 1u)] = e[i];
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < c.y; i += PR_SORT_TPB) edges[c.x + i] = o[i];
+}
+
+__global__ void __launch_bounds__(PR_PULL_TPB) k_pr_pull(const uint4 *__restrict__ chunks,
+                                                         const uint32_t *__restrict__ n_chunks,
+                                                         const uint32_t *__restrict__ edges,
+                                                         const double *__restrict__ contrib, double *acc, uint32_t V) {
+    __shared__ double sum[PR_BIN];
+    if (blockIdx.x >= *n_chunks) return;
+    const uint4 c = chunks[blockIdx.x];
+    for (uint32_t d = threadIdx.x; d < PR_BIN; d += PR_PULL_TPB) sum[d] = 0.0;
+    __syncthreads();
+    const uint32_t e0 = threadIdx.x * PR_EPT;
+    if (e0 < c.y) {
+        const uint32_t n = min(PR_EPT, c.y - e0);
+        const uint4 *ep = reinterpret_cast<const uint4 *>(edges + c.x + e0);  // chunks start at multiples of 4
+        uint32_t cur = 0xFFFFFFFFu;
+        double run = 0.0;
+        bool shared_run = true;  // the first run may go on from the thread before
+        for (uint32_t i = 0; i < n; i += 8) {
+            const uint4 a = ep[i / 4], b = i + 4 < n ? ep[i / 4 + 1] : make_uint4(0, 0, 0, 0);
+            const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            double x[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) x[q] = i + q < n ? contrib[w[q] >> PR_LOW] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                if (i + q >= n) break;
+                const uint32_t d = w[q] & (PR_BIN - 1);
+                if (d != cur) {
+                    if (cur != 0xFFFFFFFFu) {
+                        if (shared_run)
+                            atomicAdd(&sum[cur], run);
+                        else
+                            sum[cur] = run;
+                        shared_run = false;
+                    }
+                    cur = d;
+                    run = x[q];
+                } else {
+                    run += x[q];
+                }
+            }
+        }
+        atomicAdd(&sum[cur], run);  // the last run may go on in the next thread
+    }
+    __syncthreads();
+    for (uint32_t d = threadIdx.x; d < PR_BIN; d += PR_PULL_TPB) {
+        const uint32_t v = c.z * PR_BIN + d;
+        if (v >= V) break;
+        if (c.w == 1)
+            acc[v] = sum[d];
+        else if (sum[d] != 0.0)
+            atomicAdd(&acc[v], sum[d]);
+    }
+}
+
+// out-degrees from the slot ranks of the sentinels (P: exclusive prefix of
+// the segment counts), and their reciprocals
+__global__ void __launch_bounds__(TPB) k_pr_deg(const uint32_t *__restrict__ P, const uint32_t *__restrict__ sent,
+                                                uint32_t H, uint32_t V, double *inv, uint32_t *deg) {
+    for (uint64_t v = blockIdx.x * (uint64_t)TPB + threadIdx.x; v < V; v += gridDim.x * (uint64_t)TPB) {
+        const uint64_t p1 = linear_slot(sent[v], H), p0 = v ? linear_slot(sent[v - 1], H) : 0;
+        const uint32_t r1 = P[p1 >> 5] + (uint32_t)(p1 & 31), r0 = v ? P[p0 >> 5] + (uint32_t)(p0 & 31) + 1 : 0u;
+        deg[v] = r1 - r0;
+        inv[v] = r1 > r0 ? 1.0 / (double)(r1 - r0) : 0.0;
+    }
+}
+
+// rank (1/V when init, else from acc and *dangling), contrib = rank / deg,
+// the next dangling sum; clears acc and the dangling word after that
+__global__ void __launch_bounds__(TPB) k_pr_step(bool init, double *rank, double *acc, const double *__restrict__ inv,
+                                                 const uint32_t *__restrict__ deg, uint32_t V, double alpha,
+                                                 const double *__restrict__ dangling, double *next, double *after,
+                                                 double *contrib) {
+    __shared__ double ws[TPB / 32];
+    const double base = (1.0 - alpha) / (double)V, dv = init ? 0.0 : *dangling / (double)V, first = 1.0 / (double)V;
+    double d = 0;
+    for (uint64_t v = blockIdx.x * (uint64_t)TPB + threadIdx.x; v < V; v += gridDim.x * (uint64_t)TPB) {
+        const double r = init ? first : base + alpha * (acc[v] + dv);
+        rank[v] = r;
+        acc[v] = 0.0;
+        const double i = inv[v];
+        if (i == 0.0) {
+            contrib[v] = 0.0;
+            d += r;
+        } else {
+            // rank / deg from the rounded reciprocal: one correction step
+            // gives the quotient's rounding
+            const double q = r * i;
+            contrib[v] = fma(fma(-q, (double)deg[v], r), i, q);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = d;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0;
+        for (int i = 0; i < TPB / 32; i++) t += ws[i];
+        if (t != 0.0) atomicAdd(next, t);
+        if (blockIdx.x == 0) *after = 0.0;
+    }
+}
+
 __global__ void __launch_bounds__(TPB) k_fill_f64(double *p, uint64_t n, double x) {
     for (uint64_t i = blockIdx.x * (uint64_t)TPB + threadIdx.x; i < n; i += gridDim.x * (uint64_t)TPB) p[i] = x;
 }
@@ -632,6 +878,48 @@ void launch_outdeg(Geo g, const uint8_t *cnt, uint32_t *deg, cudaStream_t s) {
 
 void launch_fill_f64(double *p, uint64_t n, double x, cudaStream_t s) {
     k_fill_f64<<<grid_for(n, TPB, 152 * 8), TPB, 0, s>>>(p, n, x);
+    note_launch();
+}
+
+size_t pr_words(uint32_t V, uint64_t edges, PrLayout *l) {
+    l->nbins = (V + PR_BIN - 1) >> PR_LOW;
+    l->max_chunks = (uint32_t)(edges / PR_CHUNK) + l->nbins;
+    l->cap = (uint32_t)(edges + 4ull * l->nbins);
+    return 4ull * l->max_chunks + l->cap + l->nbins + 1;
+}
+
+cudaError_t launch_pr_layout(Geo g, const uint8_t *cnt, const uint32_t *P, const uint32_t *sent, uint32_t V,
+                             const PrLayout &l, uint32_t *words, double *inv, uint32_t *deg, cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(k_pr_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)((2 * PR_CHUNK + PR_BIN + 32) * 4));
+    if (e != cudaSuccess) return e;
+    uint4 *chunks = reinterpret_cast<uint4 *>(words);
+    uint32_t *edges = words + 4ull * l.max_chunks, *bins = edges + l.cap, *n_chunks = bins + l.nbins;
+    ProfScope ps_("pr_layout", s);
+    if ((e = cudaMemsetAsync(bins, 0, 4ull * l.nbins, s)) != cudaSuccess) return e;
+    const uint32_t tiles = (uint32_t)((nseg_of(g.H) + PR_TILE_SEGS - 1) / PR_TILE_SEGS);
+    k_pr_count<<<tiles, TPB, 0, s>>>(g, cnt, l.nbins, bins);
+    k_pr_table<<<1, 1024, 0, s>>>(l.nbins, bins, chunks, n_chunks);
+    k_pr_place<<<tiles, TPB, 0, s>>>(g, cnt, l.nbins, bins, edges, l.cap);
+    k_pr_sort<<<l.max_chunks, PR_SORT_TPB, (2 * PR_CHUNK + PR_BIN + 32) * 4, s>>>(chunks, n_chunks, edges);
+    k_pr_deg<<<grid_for(V, TPB, 152 * 8), TPB, 0, s>>>(P, sent, g.H, V, inv, deg);
+    note_launch(5);
+    return cudaGetLastError();
+}
+
+void launch_pr_pull(uint32_t it, const PrLayout &l, const uint32_t *words, uint32_t V, double alpha, const double *inv,
+                    const uint32_t *deg, double *rank, double *contrib, double *acc, double *dangling,
+                    cudaStream_t s) {
+    ProfScope ps_("pagerank", s);
+    const uint4 *chunks = reinterpret_cast<const uint4 *>(words);
+    const uint32_t *edges = words + 4ull * l.max_chunks, *n_chunks = edges + l.cap + l.nbins;
+    if (it) {
+        k_pr_pull<<<l.max_chunks, PR_PULL_TPB, 0, s>>>(chunks, n_chunks, edges, contrib, acc, V);
+        note_launch();
+    }
+    k_pr_step<<<grid_for(V, TPB, 152 * 8), TPB, 0, s>>>(it == 0, rank, acc, inv, deg, V, alpha,
+                                                        dangling + it % 3, dangling + (it + 1) % 3,
+                                                        dangling + (it + 2) % 3, contrib);
     note_launch();
 }
 

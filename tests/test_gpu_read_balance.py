@@ -2,7 +2,8 @@
 hubs whose slots fill a few segments more or less than one range of the BFS
 frontier (4 segments of 32 slots), vertices without edges, every source the
 same; neighbour lists of one query, of many, at the size up to which one CTA
-places them, and of so many that a hub's rounds are capped."""
+places them, and of so many that a hub's rounds are capped; PageRank over
+bins of 1,024 destinations and chunks of 16,384 edges."""
 import numpy as np
 import pytest
 
@@ -107,4 +108,29 @@ def test_neighbor_lists_with_capped_rounds(engine):
     wins = np.full(n, 0xFFFFF, np.uint64)
     wins[[5, n - 1]] = np.uint64(7 << 32 | 7)
     _check_lists(g, k, v, srcs, wins, V)
+    g.close()
+
+
+@pytest.mark.parametrize("V,case", [
+    (1024, "even"), (1025, "even"), (5000, "even"), (40000, "even"),  # 1, 2, 5 and 40 bins
+    (40000, "one"), (40000, "two"),  # every edge into one vertex, or into the last of a bin and the first of the next
+])
+def test_pagerank_by_destination(engine, oracle, V, case):
+    rng = np.random.default_rng(V)
+    n = 400000 if V > 2000 else 180000
+    src = rng.integers(0, V - 7, n).astype(np.uint64)  # the last vertices have no out-edges
+    if case == "even":
+        dst = rng.integers(0, V, n).astype(np.uint64)
+        dst[:100000] = rng.integers(2000 % V, 2000 % V + 40, 100000)  # one bin of several chunks
+    else:
+        dst = np.full(n, 3071, np.uint64) if case == "one" else np.where(rng.random(n) < 0.5, 3071, 3072).astype(np.uint64)
+    # a pair may be there at several times
+    keys = np.unique((src << np.uint64(42)) | (dst << np.uint64(20)) | rng.integers(0, 100000, n).astype(np.uint64))
+    assert keys.size >= 1 << 17 and 24 * keys.size >= 3 << 20  # the form under test is the one that runs
+    g = engine.Lpma(V)
+    g.update(ins=_dev(keys))
+    got = g.pagerank(0.85, 24).cpu().numpy()
+    k, _ = g.export_sorted()
+    # as test_gpu_reads: the sums' order is the only difference
+    np.testing.assert_allclose(got, oracle.pagerank(k, V, 0.85, 24), rtol=1e-10, atol=0)
     g.close()
