@@ -643,6 +643,18 @@ __device__ __forceinline__ void k_plan_body(const UpdList u, uint32_t n_cap, con
     if (threadIdx.x == 0) s_lv = 0, s_fl = 0;
     __syncthreads();
     const uint32_t nu = st->n_u;
+    // More items than a tree of one more level has slots (a bulk load into a
+    // small tree): some window overflows whatever the levels decide, and the
+    // host rebuilds the tree from the whole list, so no window is planned.
+    // The climb of every leader to the root took 900 us for 16.8M keys into a
+    // tree of 1M sentinels.
+    if (!tb.nseg) {
+        const int64_t after = (int64_t)total_live + 2 * (int64_t)st->n_ins - (int64_t)nu;
+        if (after > (int64_t)nslots_of(H + 1)) {
+            if (bid_ == 0 && threadIdx.x == 0) atomicOr(&st->ovf, 2u);
+            return;
+        }
+    }
     const uint32_t x = bid_ * TPB + threadIdx.x;
     uint32_t s = 0;
     bool lead = false;
@@ -735,8 +747,9 @@ __device__ __forceinline__ void k_plan_max_body(const Window *__restrict__ cand,
                                                   uint32_t cut_shared = SMALL_WIN_SEGS) {
     // updates of segments that no window absorbed stay pending (overflow):
     // each update copies the mark its run's first update (the planner's
-    // leader) wrote.  The marks are read only on the overflow paths.
-    if (st->ovf) {
+    // leader) wrote.  The marks are read only on the overflow paths that keep
+    // the tree's levels (bit 0; bit 1: a rebuild from the whole list).
+    if (st->ovf == 1u) {
         const uint32_t x = bid_ * TPB + threadIdx.x;
         if (x < st->n_u && x < n_cap) {
             const uint32_t s = u.seg[x];
