@@ -54,6 +54,7 @@ struct Cap {
     uint32_t *bitmap = nullptr;
     uint32_t *scan_tmp = nullptr;
     uint64_t *ts_tmp = nullptr;  // block totals of the big windows' prefix scan
+    uint32_t *done = nullptr;    // a counter of finished CTAs, 0 between kernels
     void *arena = nullptr;  // one stream-ordered allocation holding all of the above
 };
 
@@ -356,7 +357,7 @@ cudaError_t alloc_cap(Cap &c, uint32_t Hc, cudaStream_t s) {
     part(&c.segP, nseg + 2), part(&c.PQ, nseg + 2);
     part(&c.US, nseg + 2), part(&c.qi, nseg + 2), part(&c.qd, nseg + 2);
     part(&c.bitmap, bitmap_words(Hc)), part(&c.scan_tmp, scan_tmp_words((uint32_t)nseg + 2) + 64);
-    part(&c.ts_tmp, tile_prefix_tmp_words(nseg));
+    part(&c.ts_tmp, tile_prefix_tmp_words(nseg)), part(&c.done, 1);
     cudaError_t e = pool_alloc(&c.arena, off, s);
     if (e != cudaSuccess) {
         c = Cap{};
@@ -365,6 +366,7 @@ cudaError_t alloc_cap(Cap &c, uint32_t Hc, cudaStream_t s) {
     for (auto &pp : parts) *pp.first = static_cast<char *>(c.arena) + pp.second;
     if (poison_this("cap") && (e = cudaMemsetAsync(c.arena, 0xA5, off, s)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(c.cnt, 0, nseg + 64, s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(c.done, 0, sizeof(uint32_t), s)) != cudaSuccess) return e;
     return cudaMemsetAsync(c.cnt_live, 0, nseg + 64, s);
 }
 
@@ -1399,7 +1401,6 @@ lpma_status_t lpma_update_host(LpmaHandle *h, const uint64_t *h_ins, const uint8
 }
 
 static lpma_status_t fill_view(LpmaHandle *h, cudaStream_t s, bool csr, bool exp) {
-    const uint64_t nseg = nseg_of(h->H);
     const size_t nnz = h->total;
     if (csr && nnz + 1 > h->view_cap) {
         dfree(h->row_offset), dfree(h->col_index), dfree(h->view_vals);
@@ -1414,10 +1415,8 @@ static lpma_status_t fill_view(LpmaHandle *h, cudaStream_t s, bool csr, bool exp
         if (dalloc(&h->exp_keys, nnz + 1) || dalloc(&h->exp_vals, nnz + 1)) return LPMA_ERR_OUT_OF_MEMORY;
         h->exp_cap = nnz + 1;
     }
-    CK(scan_u8_to_u32(h->c.cnt, h->c.segP, (uint32_t)nseg, h->c.segP + nseg, h->c.scan_tmp, s));
-    if (csr) CK(cudaMemsetAsync(h->row_offset, 0, 4ull * (h->V + 1), s));
     Geo g{h->c.keys, h->c.vals, h->H};
-    launch_csr_fill(g, h->c.cnt, h->c.segP, csr ? h->row_offset : nullptr, csr ? h->col_index : nullptr,
+    launch_csr_fill(g, h->c.cnt, h->c.segP, h->c.done, csr ? h->row_offset : nullptr, csr ? h->col_index : nullptr,
                     csr ? h->view_vals : nullptr, exp ? h->exp_keys : nullptr, exp ? h->exp_vals : nullptr, s);
     CK(cudaGetLastError());
     return LPMA_OK;

@@ -139,8 +139,12 @@ void launch_check_empty_level(const uint8_t *cnt, uint32_t H, DevStatus *st, cud
 void launch_sum_cnt(const uint8_t *cnt, uint64_t nseg, DevStatus *st, cudaStream_t s);
 
 // view
-void launch_csr_fill(Geo g, const uint8_t *cnt, const uint32_t *P, uint32_t *row_offset, uint32_t *col_index,
-                     uint8_t *values, uint64_t *export_keys, uint8_t *export_vals, cudaStream_t s);
+// the CSR view (and / or the export) of the tree; tiles: one word per 128
+// segments and one more; done: a counter word that starts at 0 and is left
+// at 0
+void launch_csr_fill(Geo g, const uint8_t *cnt, uint32_t *tiles, uint32_t *done, uint32_t *row_offset,
+                     uint32_t *col_index, uint8_t *values, uint64_t *export_keys, uint8_t *export_vals,
+                     cudaStream_t s);
 
 // generators
 void launch_sentinels(uint32_t V, uint64_t *keys, uint8_t *vals, cudaStream_t s);

@@ -8,36 +8,164 @@ namespace {
 constexpr int TPB = 256;
 
 // to_csr_rpma (rpma.cuh:2249-2295): the present keys in linear order,
-// compacted.  One warp per segment; P is the exclusive prefix of the
-// per-segment counts, so the writes of a warp are one contiguous run.
-__global__ void __launch_bounds__(TPB) k_csr_fill(Geo g, const uint8_t *__restrict__ cnt, const uint32_t *__restrict__ P,
-                                                  uint32_t *row_offset, uint32_t *col_index, uint8_t *values,
-                                                  uint64_t *ek, uint8_t *ev) {
-    const uint64_t nseg = nseg_of(g.H);
-    const int lane = threadIdx.x & 31;
-    for (uint64_t s = (blockIdx.x * (uint64_t)TPB + threadIdx.x) >> 5; s < nseg;
-         s += (gridDim.x * (uint64_t)TPB) >> 5) {
-        const uint32_t c = cnt[s];
-        if ((uint32_t)lane >= c) continue;
-        const uint64_t j = heap_of_linear(s, g.H);
-        const uint64_t key = g.keys[32 * j + lane];
-        const uint8_t val = g.vals[32 * j + lane];
-        const uint32_t pos = P[s] + lane;
-        if (col_index) {
-            const uint32_t src = (uint32_t)(key >> SRC_SHIFT);
+// compacted.  Tiles of 128 consecutive segments: k_csr_tiles sums each
+// tile's counts, its last CTA turns the sums into starts, and one CTA of
+// k_csr_fill a tile places the columns and values in shared memory and
+// writes them out whole, 16 and 4 bytes a thread.
+//
+// Bound by HBM (9 bytes a slot read, 5 an item written).  One warp per
+// segment and one slot a lane kept too few bytes in flight and wrote 4-byte
+// words at odd places: 138 us for 18.9M items in 33.5M slots, and 16 for
+// the three kernels of its prefix; now 78 and 14.  5 CTAs a SM: 4 measured
+// 82 us, 6 (spills) 101.
+constexpr uint32_t CT = 128;                // segments a tile
+constexpr uint32_t CT_SLOTS = 32 * CT;
+constexpr int CT_TPB = 1024;  // 128 tiles a CTA, so that the last one scans 8,192 starts in one round
+
+__global__ void __launch_bounds__(CT_TPB) k_csr_tiles(const uint8_t *__restrict__ cnt, uint64_t nseg, uint32_t ntiles,
+                                                   uint32_t *tiles, uint32_t *row_offset, uint32_t *done) {
+    // 8 threads a tile, 16 counts each (the count array is padded past nseg)
+    const uint32_t t = (blockIdx.x * CT_TPB + threadIdx.x) >> 3;
+    const uint64_t s0 = (uint64_t)t * CT + 16 * (threadIdx.x & 7);
+    uint32_t c = 0;
+    if (s0 + 16 <= nseg) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(cnt + s0);
+        c = __dp4a(v.x, 0x01010101u, c);
+        c = __dp4a(v.y, 0x01010101u, c);
+        c = __dp4a(v.z, 0x01010101u, c);
+        c = __dp4a(v.w, 0x01010101u, c);
+    } else {
+        for (uint64_t s = s0; s < nseg; s++) c += cnt[s];
+    }
+    c += __shfl_xor_sync(0xffffffffu, c, 1, 8);
+    c += __shfl_xor_sync(0xffffffffu, c, 2, 8);
+    c += __shfl_xor_sync(0xffffffffu, c, 4, 8);
+    if ((threadIdx.x & 7) == 0 && t < ntiles) tiles[t] = c;
+    // the last CTA to finish: exclusive starts, 8 tiles a thread and round
+    __shared__ uint32_t last, ws[CT_TPB / 32];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1 ? 1u : 0u;  // back to 0 for the next call
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (uint32_t b0 = 0; b0 < ntiles; b0 += 8 * CT_TPB) {
+        const uint32_t i0 = b0 + 8 * threadIdx.x;
+        uint32_t x[8], sum = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < 8; q++) sum += x[q] = i0 + q < ntiles ? __ldcg(tiles + i0 + q) : 0u;
+        uint32_t v = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += y;
+        }
+        if (lane == 31) ws[w] = v;
+        __syncthreads();
+        uint32_t off = carry + v - sum;
+#pragma unroll
+        for (int k = 0; k < CT_TPB / 32; k++) {
+            const uint32_t y = ws[k];
+            off += k < w ? y : 0u;
+            carry += y;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 8; q++) {
+            if (i0 + q < ntiles) tiles[i0 + q] = off;
+            off += x[q];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        tiles[ntiles] = carry;
+        if (row_offset) row_offset[0] = 0;  // the sentinels write the others
+    }
+}
+
+__global__ void __launch_bounds__(TPB, 5) k_csr_fill(Geo g, const uint8_t *__restrict__ cnt,
+                                                  const uint32_t *__restrict__ tiles, uint32_t *row_offset,
+                                                  uint32_t *col_index, uint8_t *values, uint64_t *ek, uint8_t *ev) {
+    __shared__ __align__(16) uint32_t col[CT_SLOTS + 4];
+    __shared__ __align__(16) uint8_t val[CT_SLOTS + 4];
+    __shared__ uint32_t off[CT], ws[CT / 32];
+    const uint32_t base = tiles[blockIdx.x], tot = tiles[blockIdx.x + 1] - base;
+    if (!tot) return;
+    const uint64_t nseg = nseg_of(g.H), t0 = (uint64_t)blockIdx.x * CT;
+    const int lane = threadIdx.x & 31, gl = lane & 7, grp = threadIdx.x >> 3;
+    // the lane's slots of four segments load together
+    uint64_t k[4][4];
+    uint32_t v4[4], c[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const uint64_t s = t0 + 32 * r + grp;
+        c[r] = s < nseg ? cnt[s] : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+        if (4 * (uint32_t)gl < c[r]) {
+            const uint64_t j = heap_of_linear32((uint32_t)(t0 + 32 * r + grp), g.H);
+            const ulonglong2 *kp = reinterpret_cast<const ulonglong2 *>(g.keys + 32 * j + 4 * gl);
+            const ulonglong2 a = kp[0], b = kp[1];
+            k[r][0] = a.x, k[r][1] = a.y, k[r][2] = b.x, k[r][3] = b.y;
+            v4[r] = *reinterpret_cast<const uint32_t *>(g.vals + 32 * j + 4 * gl);
+        }
+    // where each segment's items start in the tile
+    uint32_t x = 0, v = 0;
+    if (threadIdx.x < CT) {
+        v = x = t0 + threadIdx.x < nseg ? cnt[t0 + threadIdx.x] : 0u;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += y;
+        }
+        if (lane == 31) ws[threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < CT) {
+        for (uint32_t q = 0; q < threadIdx.x >> 5; q++) v += ws[q];
+        off[threadIdx.x] = v - x;
+    }
+    __syncthreads();
+    const uint32_t sh = base & 3;  // shared position + base - sh = global position
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        if (4 * (uint32_t)gl >= c[r]) continue;
+        const uint32_t p0 = off[32 * r + grp] + 4 * gl;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (4 * (uint32_t)gl + q >= c[r]) break;
+            const uint64_t key = k[r][q];
+            const uint32_t pos = p0 + q, src = (uint32_t)(key >> SRC_SHIFT);
             const uint32_t dst = (uint32_t)((key & DST_MASK) >> DST_SHIFT);
-            if (dst == NBR_END) {
-                col_index[pos] = src;
-                values[pos] = VAL_TOMB;
-                row_offset[src + 1] = pos + 1;
-            } else {
-                col_index[pos] = dst;
-                values[pos] = val;
+            const bool end = dst == NBR_END;
+            const uint8_t vq = (uint8_t)(v4[r] >> (8 * q));
+            if (col_index) {
+                col[sh + pos] = end ? src : dst;
+                val[sh + pos] = end ? VAL_TOMB : vq;
+                if (end) row_offset[src + 1] = base + pos + 1;
+            }
+            if (ek) {
+                ek[base + pos] = key;
+                ev[base + pos] = vq;
             }
         }
-        if (ek) {
-            ek[pos] = key;
-            ev[pos] = val;
+    }
+    if (!col_index) return;
+    __syncthreads();
+    // shared words [sh, sh + tot): whole vectors, the ends by element
+    const uint32_t e = sh + tot, v0 = (sh + 3) / 4, v1 = e / 4, at = base - sh;
+    for (uint32_t i = v0 + threadIdx.x; i < v1; i += TPB) {
+        reinterpret_cast<uint4 *>(col_index + at)[i] = reinterpret_cast<const uint4 *>(col)[i];
+        reinterpret_cast<uint32_t *>(values + at)[i] = reinterpret_cast<const uint32_t *>(val)[i];
+    }
+    const uint32_t head = min(4 * v0, e), tail = max(4 * v1, head);
+    if (threadIdx.x < 8) {
+        const uint32_t i = threadIdx.x < 4 ? sh + threadIdx.x : tail + threadIdx.x - 4;
+        if (i < (threadIdx.x < 4 ? head : e)) {
+            col_index[at + i] = col[i];
+            values[at + i] = val[i];
         }
     }
 }
@@ -96,12 +224,18 @@ inline uint32_t grid_for(uint64_t n, uint32_t per_block, uint32_t cap = 152 * 16
 
 }  // namespace
 
-void launch_csr_fill(Geo g, const uint8_t *cnt, const uint32_t *P, uint32_t *row_offset, uint32_t *col_index,
-                     uint8_t *values, uint64_t *export_keys, uint8_t *export_vals, cudaStream_t s) {
+void launch_csr_fill(Geo g, const uint8_t *cnt, uint32_t *tiles, uint32_t *done, uint32_t *row_offset,
+                     uint32_t *col_index, uint8_t *values, uint64_t *export_keys, uint8_t *export_vals,
+                     cudaStream_t s) {
+    const uint64_t nseg = nseg_of(g.H);
+    const uint32_t ntiles = (uint32_t)((nseg + CT - 1) / CT);
+    {
+        ProfScope ps_("csr_tiles", s);
+        k_csr_tiles<<<(ntiles + CT_TPB / 8 - 1) / (CT_TPB / 8), CT_TPB, 0, s>>>(cnt, nseg, ntiles, tiles, row_offset, done);
+    }
     ProfScope ps_("csr_fill", s);
-    k_csr_fill<<<grid_for(nseg_of(g.H), TPB / 32), TPB, 0, s>>>(g, cnt, P, row_offset, col_index, values, export_keys,
-                                                                export_vals);
-    note_launch();
+    k_csr_fill<<<ntiles, TPB, 0, s>>>(g, cnt, tiles, row_offset, col_index, values, export_keys, export_vals);
+    note_launch(2);
 }
 
 void launch_sentinels(uint32_t V, uint64_t *keys, uint8_t *vals, cudaStream_t s) {

@@ -134,3 +134,24 @@ def test_pagerank_by_destination(engine, oracle, V, case):
     # as test_gpu_reads: the sums' order is the only difference
     np.testing.assert_allclose(got, oracle.pagerank(k, V, 0.85, 24), rtol=1e-10, atol=0)
     g.close()
+
+
+@pytest.mark.parametrize("V,n", [(1, 0), (31, 40), (96, 30), (97, 900), (200, 4000), (1500, 25000), (70000, 3000)])
+def test_csr_view_tile_edges(engine, oracle, V, n):
+    """Views of 1 to a few hundred tiles of 128 segments, whose starts fall on
+    every remainder of the 16-byte stores."""
+    from test_gpu_parity import assert_csr
+    rng = np.random.default_rng(V)
+    g, o = engine.Lpma(V), oracle.OracleLpma(V)
+    for step in range(4):
+        i = rng.permutation(V * V * 64)[:n + step].astype(np.uint64) if V < 1600 else rng.integers(0, 1 << 40, n + step).astype(np.uint64)
+        keys = ((i % np.uint64(V)) << np.uint64(42)) | ((i // np.uint64(V) % np.uint64(V)) << np.uint64(20)) | \
+            (i // np.uint64(V) // np.uint64(V) % np.uint64(1 << 20))
+        keys = np.unique(keys)
+        vals = rng.integers(1, 255, keys.size).astype(np.uint8)
+        if keys.size:
+            import torch
+            g.update(ins=_dev(keys), ins_vals=torch.from_numpy(vals).cuda())
+            o.update(ins=keys, ins_vals=vals)
+        assert_csr(g, o)
+    g.close()
