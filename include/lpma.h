@@ -95,7 +95,8 @@ typedef struct {
     uint64_t h2d_bytes;        /* host->device bytes the call copied (inputs, control) */
     uint64_t d2h_bytes;        /* device->host bytes the call copied (status blocks) */
     uint32_t sort_passes;      /* digit passes the batch sort ran: one per byte that varies over the batch,
-                                  or, for the cooperative sort, one per 9-bit digit window */
+                                  or, for the cooperative sort, one per 9-bit digit window; 1 for the
+                                  partitioned front, which sorts by place in the tree in one pass */
     uint32_t levelup;          /* update_rpma's return value (rpma.cuh:1646-1653, 1662-1668): 1 when updates
                                   reached the root level, i.e. the root window absorbed them (root_executed,
                                   whether or not a level was added) or they overflowed it (overflow, whatever
@@ -297,7 +298,11 @@ LPMA_API lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *grap
                                          size_t n, lpma_stream_t stream, LpmaStats *stats, lpma_status_t *status);
 
 /* ---- autotuner: the batch-sort algorithm per batch-size bucket ----
- * The update front sorts each batch with one of five algorithms ("tiers"):
+ * Batches of 256 to 2^21 keys on trees of height 9 and more take the
+ * partitioned front, which does not sort the whole batch, unless they
+ * crowd into one of its buckets; lpma_tune_set with a tier other than 0
+ * keeps the batches of its entry off it.  The sorted front sorts each batch
+ * with one of five algorithms ("tiers"):
  * 1 one CTA through shared memory (<= 2048 keys), 2 tiles of 2048 keys
  * sorted by all-pairs rank over many CTAs, then placed by binary searches
  * across the tiles (<= 16384), 3 register-sorted tiles plus

@@ -54,6 +54,7 @@ struct Cap {
     uint32_t *bitmap = nullptr;
     uint32_t *scan_tmp = nullptr;
     uint64_t *ts_tmp = nullptr;  // block totals of the big windows' prefix scan
+    uint32_t *absbits = nullptr; // the partitioned front's executed segments (bit s + 1)
     uint32_t *done = nullptr;    // a counter of finished CTAs, 0 between kernels
     void *arena = nullptr;  // one stream-ordered allocation holding all of the above
 };
@@ -149,6 +150,15 @@ struct LpmaHandle {
     // cached front graphs hold raw pointers to every such buffer, so they
     // are all dropped when one moves.  (The sort mode is part of their key.)
     uint64_t buf_gen = 1, graph_gen = 0;
+    // the partitioned front (front.cu): bucket entries, per-bucket words
+    // (fill counts, zero between calls; updates left; windows executed)
+    ulonglong2 *part_ent = nullptr;
+    size_t part_cap = 0;  // entries
+    uint32_t *part_ctl = nullptr;
+    bool front_part = false;  // the last front was the partitioned one
+    // calls to go before the partitioned front is tried again after a batch
+    // whose buckets overflowed (its keys crowd into a part of the tree)
+    uint32_t part_skip = 0;
     // the last front sorted with the cooperative sort's 9-bit digits (for
     // the pass count in the stats)
     bool front_sort_wide = false;
@@ -165,6 +175,10 @@ namespace {
 bool pagerank_pulls(uint64_t edges, uint32_t iterations) {
     return iterations >= 3 && edges >= (1u << 17) && edges * iterations >= (3u << 20);
 }
+
+// calls on the sorted front after a batch whose buckets overflowed: a stream
+// of such batches pays the vain partition (about 30 us) once in 17 calls
+constexpr uint32_t PART_SKIP = 16;
 
 // levels of a BFS launched before the host reads their counters back, the
 // counters of those levels (ranges and vertices of each frontier), and the
@@ -358,6 +372,7 @@ cudaError_t alloc_cap(Cap &c, uint32_t Hc, cudaStream_t s) {
     part(&c.US, nseg + 2), part(&c.qi, nseg + 2), part(&c.qd, nseg + 2);
     part(&c.bitmap, bitmap_words(Hc)), part(&c.scan_tmp, scan_tmp_words((uint32_t)nseg + 2) + 64);
     part(&c.ts_tmp, tile_prefix_tmp_words(nseg)), part(&c.done, 1);
+    part(&c.absbits, bitmap_words(Hc));
     cudaError_t e = pool_alloc(&c.arena, off, s);
     if (e != cudaSuccess) {
         c = Cap{};
@@ -486,7 +501,7 @@ bool needs_prefix(const Tables &tb, uint32_t H) {
 // first plan), so no memset sits between the front's kernels
 lpma_status_t run_plan(LpmaHandle *h, const UpdList &u, uint32_t n_cap, bool thres_active, uint64_t total_live,
                        const Tables &tb, cudaStream_t s, const unsigned long long *total_live_dev = nullptr,
-                       bool fresh = false, DevStatus *pub = nullptr) {
+                       bool fresh = false, DevStatus *pub = nullptr, const BucketArgs *part = nullptr) {
     const uint32_t H = h->H;
     const uint64_t nseg = nseg_of(H);
     if (!fresh) {
@@ -497,7 +512,7 @@ lpma_status_t run_plan(LpmaHandle *h, const UpdList &u, uint32_t n_cap, bool thr
     const bool useP = needs_prefix(tb, H);
     if (useP) CK(scan_u8_to_u32(cntp, h->c.segP, (uint32_t)nseg, h->c.segP + nseg, h->c.scan_tmp, s));
     launch_plan(u, n_cap, cntp, h->c.segP, useP ? 1 : 0, total_live, total_live_dev, H, tb, h->c.bitmap, h->cand,
-                h->wsingle, h->wsmall4, h->wsmall, h->wbig, h->pend, h->dst, s, pub);
+                h->wsingle, h->wsmall4, h->wsmall, h->wbig, h->pend, h->dst, s, pub, part);
     CK(cudaGetLastError());
     return LPMA_OK;
 }
@@ -527,10 +542,13 @@ lpma_status_t exec_plan(LpmaHandle *h, const UpdList &u, uint32_t n_list, uint32
         launch_exec_multi(h->wsmall4, n_small4, h->wsmall, n_small, g, h->c.cnt, h->c.fl, h->sent, h->V, u, thres,
                           h->dst, s);
     }
-    st->windows_single += n_single;
-    st->windows_small += n_single + n_small4 + n_small;
-    st->slots_rewritten += h->hst->slots_small;
-    st->slots_small += h->hst->slots_small;
+    // single-segment windows that the partitioned front executed and no
+    // larger window covers
+    const uint64_t n_abs = h->hst->abs_win - h->hst->abs_hidden;
+    st->windows_single += n_single + n_abs;
+    st->windows_small += n_single + n_small4 + n_small + n_abs;
+    st->slots_rewritten += h->hst->slots_small + 32 * n_abs;
+    st->slots_small += h->hst->slots_small + 32 * n_abs;
     if (n_big) {
         // the job list is built on the device (windows sorted by position,
         // tile prefix); the tile count came with the status read-back, so
@@ -685,6 +703,74 @@ lpma_status_t enqueue_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, 
     return LPMA_OK;
 }
 
+// The partitioned front of a batch, up to the status read-back and the
+// executors of the windows that its list plans.
+lpma_status_t enqueue_part(LpmaHandle *h, cudaStream_t s, const PartArgs &pa, size_t n, const PartPlan &pp,
+                           bool thres_active) {
+    CK(cudaMemcpyAsync(h->dst, h->hinit, offsetof(DevStatus, sticky), cudaMemcpyHostToDevice, s));
+    launch_part(pa, s);
+    if (thres_active) launch_live_counts(h->c.keys, h->H, pa.thres, h->c.cnt_live, h->dst, s);
+    Tables tb = make_tables(h, h->H, true);
+    set_grain(tb, n);
+    const Geo g{h->c.keys, h->c.vals, h->H};
+    const BucketArgs ba{g, h->c.fl, h->c.cnt, thres_active ? h->c.cnt_live : nullptr, h->sent, h->V, pa.thres,
+                        tb.lower[0], pp.L, pp.cap, h->part_ent, pa.fill, pa.fill + (1u << PART_L_MAX),
+                        pa.fill + (2u << PART_L_MAX), h->c.absbits, h->dst};
+    launch_buckets(ba, h->u, s);
+    const bool pub = front_publishes(h);
+    CKS(run_plan(h, h->u, (uint32_t)n, thres_active, 0, tb, s,
+                 thres_active ? &h->dst->live_total : &h->dst->total_items, true, pub ? h->hst_dev : nullptr, &ba));
+    // the status copy (or the event that backs the poll) on a branch, the
+    // executor behind the planner; no window of one segment is left
+    const bool fork = !prof_enabled();
+    cudaStream_t side = fork ? h->side_stream : s;
+    if (fork) {
+        CK(cudaEventRecord(h->fork_ev, s));
+        CK(cudaStreamWaitEvent(side, h->fork_ev, 0));
+    }
+    if (!pub) CK(cudaMemcpyAsync(h->hst, h->dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, side));
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &cs));
+    CK(cudaEventRecordWithFlags(blocking_waits(h) ? h->front_ev_blk : h->front_ev, side,
+                                cs == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault));
+    if (fork) CK(cudaEventRecord(h->join_ev, side));
+    launch_exec_multi(h->wsmall4, (uint32_t)n, h->wsmall, (uint32_t)n, g, h->c.cnt, h->c.fl, h->sent, h->V, h->u,
+                      pa.thres, h->dst, s, true);
+    if (fork) CK(cudaStreamWaitEvent(s, h->join_ev, 0));
+    return LPMA_OK;
+}
+
+// The partitioned front's plan for a batch (L = 0: the sorted front): not
+// for the engine's own sentinels, a sort tier set by the caller, or a handle
+// whose buckets overflowed lately.
+PartPlan plan_part(LpmaHandle *h, size_t n, bool internal) {
+    if (internal || h->part_skip || sort_tier_forced((uint32_t)n, h->sort)) return PartPlan{0, 0, 0};
+    return part_plan(n, h->H);
+}
+
+lpma_status_t ensure_part(LpmaHandle *h, const PartPlan &pp, cudaStream_t s) {
+    if (!h->part_ctl) {
+        CK(dalloc(&h->part_ctl, 3u << PART_L_MAX));
+        CK(cudaMemsetAsync(h->part_ctl, 0, 4u << PART_L_MAX, s));
+        CK(part_prepare());
+        h->buf_gen++;
+    }
+    const size_t need = (size_t)pp.cap << pp.L;
+    if (need <= h->part_cap) return LPMA_OK;
+    h->buf_gen++;
+    size_t cap = 1u << 14;
+    while (cap < need) cap <<= 1;
+    h->part_cap = 0;
+    if (h->part_ent) {
+        CK(cudaFreeAsync(h->part_ent, s));
+        h->part_ent = nullptr;
+    }
+    CK(pool_alloc((void **)&h->part_ent, cap * sizeof(ulonglong2), s));
+    if (poison_this("part")) CK(cudaMemsetAsync(h->part_ent, 0xA5, cap * sizeof(ulonglong2), s));
+    h->part_cap = cap;
+    return LPMA_OK;
+}
+
 bool graphs_enabled() {
     static int on = -1;
     if (on < 0) {
@@ -705,15 +791,24 @@ lpma_status_t run_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, cons
     // the stored-key count reaches the planner through the status reset copy,
     // so that it is not a kernel argument of a cached graph
     h->hinit->total_items = h->total;
-    h->front_sort_wide = update_sort_mask(nullptr, sort_tier_for_update((uint32_t)n, h->sort), (uint32_t)n, h->sort).wide;
+    const PartPlan pp = plan_part(h, n, internal);
+    h->front_part = pp.L != 0;
+    if (pp.L) CKS(ensure_part(h, pp, s));
+    const PartArgs pa{ins, ins_vals, del, (uint32_t)n_ins, (uint32_t)n_del, h->V, thres, h->cfg.key_format, pp.L, pp.cap,
+                      pp.ipt, h->c.fl, h->part_ent, h->part_ctl, h->c.bitmap, (uint32_t)bitmap_words(h->H), h->dst};
+    auto enqueue = [&](cudaStream_t st) {
+        return pp.L ? enqueue_part(h, st, pa, n, pp, thres_active)
+                    : enqueue_front(h, st, ins, ins_vals, n_ins, del, n_del, thres, thres_active, internal);
+    };
+    h->front_sort_wide = !pp.L && update_sort_mask(nullptr, sort_tier_for_update((uint32_t)n, h->sort), (uint32_t)n, h->sort).wide;
     if (internal || prof_enabled() || !graphs_enabled()) {
-        CKS(enqueue_front(h, s, ins, ins_vals, n_ins, del, n_del, thres, thres_active, internal));
+        CKS(enqueue(s));
     } else {
         const uint64_t key[12] = {n_ins, n_del, h->H, thres,
                                   (uint64_t)thres_active | ((uint64_t)(ins_vals != nullptr) << 1) |
                                       ((uint64_t)(h->sort.bar != nullptr) << 2) |
                                       ((uint64_t)sort_tier_for_update((uint32_t)n, h->sort) << 3) |
-                                      ((uint64_t)grain_word(n) << 16),
+                                      ((uint64_t)grain_word(n) << 16) | ((uint64_t)pp.L << 32) | ((uint64_t)pp.cap << 40),
                                   (uint64_t)h->c.keys, (uint64_t)h->c.vals, (uint64_t)h->c.cnt, (uint64_t)h->c.fl,
                                   (uint64_t)h->bk0, (uint64_t)h->c.cnt_live, (uint64_t)h->c.bitmap};
         if (h->graph_gen != h->buf_gen) {
@@ -736,7 +831,7 @@ lpma_status_t run_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, cons
             for (uint64_t x : h->recent_shapes) seen |= x == hk;
             if (!seen) {
                 h->recent_shapes[h->recent_pos++ % 8] = hk;
-                return enqueue_front(h, s, ins, ins_vals, n_ins, del, n_del, thres, thres_active, internal);
+                return enqueue(s);
             }
         }
         if (!fg) {
@@ -751,8 +846,7 @@ lpma_status_t run_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, cons
             memcpy(f.key, key, sizeof(key));
             const uint64_t l0 = launch_count();
             CK(cudaStreamBeginCapture(h->cap_stream, cudaStreamCaptureModeThreadLocal));
-            lpma_status_t r = enqueue_front(h, h->cap_stream, ins, ins_vals, n_ins, del, n_del, thres, thres_active,
-                                            internal);
+            lpma_status_t r = enqueue(h->cap_stream);
             cudaGraph_t gr = nullptr;
             cudaError_t ce = cudaStreamEndCapture(h->cap_stream, &gr);
             if (r != LPMA_OK) return r;
@@ -770,7 +864,7 @@ lpma_status_t run_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, cons
                 if (t != cudaGraphNodeTypeKernel) continue;
                 cudaKernelNodeParams kp;
                 CK(cudaGraphKernelNodeGetParams(nd, &kp));
-                if (kp.func == pack_kernel_fn()) {
+                if (kp.func == (pp.L ? part_kernel_fn() : pack_kernel_fn())) {
                     f.pack = nd;
                     f.pack_params = kp;
                 }
@@ -799,10 +893,12 @@ lpma_status_t run_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, cons
         uint32_t *a_sup = h->sup;
         uint32_t a_supw = sup_words_for(n);
         uint32_t *a_bar = h->sort.bar;
+        PartArgs a_part = pa;
+        void *part_args[] = {&a_part};  // k_part(PartArgs)
         void *args[] = {&a_ins, &a_vals, &a_nins, &a_del, &a_ndel, &a_V, &a_thres, &a_fmt, &a_internal, &a_ko, &a_po, &a_st,
                         &a_bm, &a_bmw, &a_fl, &a_cnt, &a_pf, &a_sup, &a_supw, &a_bar};
         cudaKernelNodeParams kp = fg->pack_params;
-        kp.kernelParams = args;
+        kp.kernelParams = pp.L ? part_args : args;
         kp.extra = nullptr;
         CK(cudaGraphExecKernelNodeSetParams(fg->exec, fg->pack, &kp));
         CK(cudaGraphLaunch(fg->exec, s));
@@ -861,7 +957,9 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
         // the digit passes the sort made: one per differing byte, or with
         // 9-bit digits one per window (the greedy plan of the sort itself)
         uint64_t diff = h->hst->key_and ^ h->hst->key_or;
-        if (h->front_sort_wide) {
+        if (h->front_part) {
+            st.sort_passes = 1;  // the partition
+        } else if (h->front_sort_wide) {
             while (diff) {
                 const int b = __builtin_ctzll(diff);
                 diff = b + WIDE_DIGIT_BITS >= 64 ? 0ull : (diff >> (b + WIDE_DIGIT_BITS)) << (b + WIDE_DIGIT_BITS);
@@ -872,8 +970,12 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
         }
     }
     const uint32_t min_t_ins = h->hst->min_t_ins;
-    const int64_t live_before = thres_active ? (int64_t)h->hst->live_total : (int64_t)h->total;
-    const uint32_t n_u = h->hst->n_u, n_new = h->hst->n_ins, n_gone = h->hst->n_del;
+    // (live_total holds the windows that the partitioned front executed)
+    const int64_t live_before = thres_active ? (int64_t)h->hst->live_total - (int64_t)h->hst->abs_ins + (int64_t)h->hst->abs_del
+                                             : (int64_t)h->total;
+    // the list's updates and those of the windows that the partitioned front
+    // executed already
+    const uint32_t n_u = h->hst->n_u, n_new = h->hst->n_ins + h->hst->abs_ins, n_gone = h->hst->n_del + h->hst->abs_del;
     st.n_ins_applied = n_new;
     st.n_del_applied = n_gone;
     st.n_upserts = h->hst->n_upsert;
@@ -881,7 +983,7 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
     const int64_t live_after = live_before - n_gone + n_new;
 
     lpma_status_t r = LPMA_OK;
-    if (n_u > 0 && !h->hst->ovf) {
+    if (n_new + n_gone > 0 && !h->hst->ovf) {
         const bool root = h->hst->root != 0;
         r = exec_plan(h, h->u, (uint32_t)n, thres, thres_active, s, &st, small_done);
         if (r == LPMA_OK && root) {
@@ -989,7 +1091,16 @@ lpma_status_t do_update(LpmaHandle *h, const uint64_t *ins, const uint8_t *ins_v
     // batch shape repeats), then the one host round trip of the common path;
     // a rejected batch turns every kernel after k_pack into a no-op
     CKS(run_front(h, s, ins, ins_vals, n_ins, del, n_del, thres, thres_active, internal));
-    return finish_update(h, wait_front(h, s), n, thres, thres_active, s, st, out, true);
+    lpma_status_t rs = wait_front(h, s);
+    if (h->part_skip) h->part_skip--;
+    if (rs == LPMA_OK && h->hst->part_ovf && !(h->hst->error & ERR_KEY)) {
+        // a bucket overflowed and nothing was done: the sorted front takes
+        // this batch, and the next ones for a while
+        h->part_skip = PART_SKIP;
+        CKS(run_front(h, s, ins, ins_vals, n_ins, del, n_del, thres, thres_active, internal));
+        rs = wait_front(h, s);
+    }
+    return finish_update(h, rs, n, thres, thres_active, s, st, out, true);
 }
 
 }  // namespace
@@ -1213,6 +1324,7 @@ lpma_status_t lpma_destroy(LpmaHandle *h) {
     h->arena = nullptr;
     dfree_async(h->sort.hist), dfree_async(h->sort.counters), dfree_async(h->sort_err);
     dfree_async(h->jobs_d);
+    dfree_async(h->part_ent), dfree_async(h->part_ctl);
     for (int b = 0; b < 2; b++) {
         dfree_async(h->stage_ins[b]), dfree_async(h->stage_del[b]), dfree_async(h->stage_vals[b]);
         if (h->stage_free[b]) cudaEventDestroy(h->stage_free[b]);
@@ -1725,7 +1837,7 @@ lpma_status_t lpma_memory_bytes(const LpmaHandle *h, uint64_t *bytes) {
         const uint64_t ns = nslots_of(h->c.Hc), nseg = nseg_of(h->c.Hc);
         b += 18 * ns + nseg * (4 + 16 + 7 * 4) + bitmap_words(h->c.Hc) * 4;
     }
-    b += 4ull * h->V + h->bcap * 64ull + h->view_cap * 9ull + h->exp_cap * 9ull + h->stage_cap * 34ull;
+    b += 4ull * h->V + h->bcap * 64ull + h->part_cap * 16ull + h->view_cap * 9ull + h->exp_cap * 9ull + h->stage_cap * 34ull;
     b += h->bfs_cap * 16ull;
     if (h->pr_deg) b += 20ull * h->V;
     b += h->q_cap * 12ull;
@@ -1939,6 +2051,7 @@ lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *graphs, const
                                                        : ((e & ERR_INTERNAL) ? LPMA_ERR_INTERNAL : LPMA_OK);
             sts[i].height_before = h->H;
             h->front_sort_wide = false;  // the shared tile-merge sort
+            h->front_part = false;
             res[i] = finish_update(h, rs, items[i].n_ins + items[i].n_del, 0, false, st, sts[i], &sts[i],
                                    shared[k] != 0);
         };
@@ -2058,7 +2171,7 @@ lpma_status_t lpma_debug_exec_wait(int give_up) {
 
 lpma_status_t lpma_tune_set(uint32_t log2_keys, uint32_t concurrent, uint32_t tier) {
     if (log2_keys > 32 || tier >= TIER_COUNT) return LPMA_ERR_INVALID_ARGUMENT;
-    sort_tier_set(log2_keys, concurrent ? 1 : 0, (SortTier)tier);
+    sort_tier_set(log2_keys, concurrent ? 1 : 0, (SortTier)tier, true);
     return LPMA_OK;
 }
 
@@ -2260,7 +2373,7 @@ lpma_status_t lpma_autotune(uint32_t max_keys, lpma_stream_t stream, LpmaTuneEnt
             if (r == LPMA_OK && (cudaMemcpy(&herr, err, 4, cudaMemcpyDeviceToHost) || herr)) r = LPMA_ERR_TIMEOUT;
             if (r != LPMA_OK) break;
             ent.tier = best_t;
-            sort_tier_set(b, conc, (SortTier)best_t);
+            sort_tier_set(b, conc, (SortTier)best_t, false);
             if (out && nout < cap) out[nout] = ent;
             nout++;
         }

@@ -42,6 +42,49 @@ inline uint32_t sup_words_for(uint64_t n) { return 2 * (uint32_t)((n + 256 * 64 
 // the pack kernel's entry (graph replays update its input pointers)
 const void *pack_kernel_fn();
 
+// ---- the partitioned front (front.cu): buckets by subtree, then located,
+// ordered, resolved and single-segment windows executed bucket by bucket
+constexpr uint32_t PART_L_MAX = 11, PART_IPT = 8;
+constexpr uint64_t PART_MIN = 256, PART_MAX = 1u << 21;  // keys of a batch
+struct PartPlan {
+    uint32_t L;    // 2^L buckets; 0: the sorted front takes the batch
+    uint32_t cap;  // entries of a bucket
+    uint32_t ipt;  // keys a thread of the partition takes
+};
+PartPlan part_plan(uint64_t n, uint32_t H);
+struct PartArgs {
+    const uint64_t *ins;
+    const uint8_t *ins_vals;
+    const uint64_t *del;
+    uint32_t n_ins, n_del, V, thres, key_format;
+    uint32_t L, cap, ipt;
+    const ulonglong2 *fl;
+    ulonglong2 *ent;  // 2^L buckets of cap entries (key, payload)
+    uint32_t *fill;   // entries of each bucket (zero before)
+    uint32_t *bitmap;
+    uint32_t bitmap_words;
+    DevStatus *st;
+};
+struct BucketArgs {
+    Geo g;
+    ulonglong2 *fl;
+    uint8_t *cnt, *cnt_live;  // cnt_live: with an active expiry threshold, else null
+    uint32_t *sent;
+    uint32_t V, thres, lower0, L, cap;
+    ulonglong2 *ent;
+    uint32_t *fill;
+    uint32_t *pcnt;     // per bucket: updates left (low half) and inserts among them
+    uint32_t *bwin;     // per bucket: single-segment windows executed
+    uint32_t *absbits;  // bit s + 1: segment s was executed
+    DevStatus *st;
+};
+// the partition kernel's entry (graph replays replace its arguments)
+const void *part_kernel_fn();
+cudaError_t part_prepare();  // once per device, outside capture
+void launch_part(const PartArgs &a, cudaStream_t s);
+// the buckets, then what is left into the update list
+void launch_buckets(const BucketArgs &a, const UpdList &u, cudaStream_t s);
+
 // per-segment live counts (key present and t >= thres) + their total
 void launch_live_counts(const uint64_t *keys, uint32_t H, uint32_t thres, uint8_t *cnt_live, DevStatus *st,
                         cudaStream_t s);
@@ -76,11 +119,14 @@ cudaError_t set_exec_wait_debug(uint32_t give_up);
 // count-only planner: per segment with updates, the first level whose
 // window passes the density test; maximal windows go to small/big lists.
 // pub: when set, the planner's last CTA writes the status block into this
-// pinned host mirror and then sets its `published` word.
+// pinned host mirror and then sets its `published` word.  part: set by the
+// partitioned front, whose list is short: a smaller grid loops over it, and
+// the single-segment windows that larger ones cover are counted.
 void launch_plan(const UpdList u, uint32_t n_cap, const uint8_t *cnt, const uint32_t *P, int use_P,
                  uint64_t total_live, const unsigned long long *total_live_dev, uint32_t H, const Tables &tb,
                  uint32_t *bitmap, Window *cand, Window *single, Window *small4, Window *small, Window *big,
-                 uint8_t *pend, DevStatus *st, cudaStream_t s, DevStatus *pub = nullptr);
+                 uint8_t *pend, DevStatus *st, cudaStream_t s, DevStatus *pub = nullptr,
+                 const BucketArgs *part = nullptr);
 
 // in-place executors for windows of <= 32 segments: the single-segment
 // list (DevStatus::n_single), and in one launch the windows of 2..4

@@ -88,6 +88,8 @@ struct DevStatus {
     uint32_t n_ins, n_del, n_upsert, n_noop;
     uint32_t n_cand, n_single, n_small4, n_small, n_big;
     uint32_t big_tiles;       // 32-segment tiles of the big windows
+    uint32_t abs_win;         // single-segment windows that the partitioned front executed
+    uint32_t abs_hidden;      // of which inside a larger executed window
     uint32_t root, ovf;
     uint32_t exec_levels;     // bit l: some window of level l executes
     uint32_t empty_found;     // fill_empty_segs check
@@ -96,6 +98,8 @@ struct DevStatus {
     unsigned long long cnt_total;    // sum of occupancy counts (recount)
     unsigned long long total_items;  // keys stored before the call (set by the host)
     uint32_t err_info[4];            // first offending input index, internal-check site
+    uint32_t abs_ins, abs_del;       // inserts and deletes of the abs_win windows
+    uint32_t part_ovf;               // a bucket overflowed: nothing was done, the sorted front takes the batch
     uint32_t plan_done;              // planner CTAs finished (the front's status publish)
     // Not reset per call (the reset copies the fields above only): the
     // executors set ERR_INTERNAL here after the call may have returned.

@@ -1481,7 +1481,7 @@ cudaError_t sort_pairs(uint64_t *k0, V *v0, uint64_t *k1, V *v1, uint32_t n, uin
 }
 
 SortTier sort_tier_for_update(uint32_t n, const SortScratch &s) {
-    const uint32_t t = g_tier_table[s.bar ? 1 : 0][log2_bucket(n)].load(std::memory_order_relaxed);
+    const uint32_t t = g_tier_table[s.bar ? 1 : 0][log2_bucket(n)].load(std::memory_order_relaxed) & 0x7F;
     if (t && tier_ok<uint16_t>((SortTier)t, n, s)) return (SortTier)t;
     return tier_default<uint16_t>(n, s);
 }
@@ -1495,12 +1495,21 @@ SortMask update_sort_mask(const unsigned long long *andor, SortTier t, uint32_t 
     return SortMask{andor, 0xFFu, pp, wide ? 1u : 0u};
 }
 
-void sort_tier_set(uint32_t bucket, int concurrent, SortTier t) {
-    if (bucket < 33) g_tier_table[concurrent ? 0 : 1][bucket].store((uint8_t)t, std::memory_order_relaxed);
+// forced: set by the caller (lpma_tune_set), not by the tuner's measurement
+constexpr uint8_t TIER_FORCED = 0x80;
+
+void sort_tier_set(uint32_t bucket, int concurrent, SortTier t, bool forced) {
+    if (bucket < 33)
+        g_tier_table[concurrent ? 0 : 1][bucket].store((uint8_t)(t | (forced && t ? TIER_FORCED : 0)),
+                                                       std::memory_order_relaxed);
+}
+
+bool sort_tier_forced(uint32_t n, const SortScratch &s) {
+    return (g_tier_table[s.bar ? 1 : 0][log2_bucket(n)].load(std::memory_order_relaxed) & TIER_FORCED) != 0;
 }
 
 SortTier sort_tier_get(uint32_t bucket, int concurrent) {
-    return bucket < 33 ? (SortTier)g_tier_table[concurrent ? 0 : 1][bucket].load(std::memory_order_relaxed) : TIER_AUTO;
+    return bucket < 33 ? (SortTier)(g_tier_table[concurrent ? 0 : 1][bucket].load(std::memory_order_relaxed) & 0x7F) : TIER_AUTO;
 }
 
 template <typename V>

@@ -66,7 +66,10 @@ bool sort_tier_usable(SortTier t, uint32_t n, const SortScratch &s);
 // words andor (AND, OR of the keys), ping-pong parity for the ping-pong
 // tiers, 9-bit digits for the cooperative tier when its scratch allows.
 SortMask update_sort_mask(const unsigned long long *andor, SortTier t, uint32_t n, const SortScratch &s);
-void sort_tier_set(uint32_t bucket, int concurrent, SortTier t);
+// forced: the caller asks for this sort (the partitioned front, which sorts
+// no batch, then leaves such batches to it); else a tuner's measurement
+void sort_tier_set(uint32_t bucket, int concurrent, SortTier t, bool forced);
+bool sort_tier_forced(uint32_t n, const SortScratch &s);
 SortTier sort_tier_get(uint32_t bucket, int concurrent);
 
 // Which digit bytes a sort pass must handle: either fixed by the host, or

@@ -734,7 +734,46 @@ __global__ void __launch_bounds__(TPB) k_plan(const UpdList u, uint32_t n_cap, c
                                               Tables tb, uint32_t *bitmap, Window *cand, uint8_t *pend,
                                               DevStatus *st) {
     griddep_wait();
-    k_plan_body(u, n_cap, cnt, P, use_P, total_live_host, total_live_dev, H, tb, bitmap, cand, pend, st, blockIdx.x, gridDim.x);
+    // one chunk of the list a block; after the partitioned front the list is
+    // short against its bound, so the grid is small and loops
+    const uint32_t nu = min(st->n_u, n_cap);
+    uint32_t c = blockIdx.x;
+    do {
+        k_plan_body(u, n_cap, cnt, P, use_P, total_live_host, total_live_dev, H, tb, bitmap, cand, pend, st, c, gridDim.x);
+        c += gridDim.x;
+    } while ((uint64_t)c * TPB < nu);
+}
+
+// How many of the segments [a, a + f) the partitioned front executed (bit
+// s + 1 of bits; bwin: per bucket of W segments, bit b W on), summed by a
+// warp: whole buckets by their counts, the ends by their bits.
+struct Absorbed {
+    const uint32_t *bits, *bwin;
+    uint32_t W;
+};
+__device__ __forceinline__ uint32_t abs_bits(const uint32_t *bits, uint32_t lo, uint32_t hi, uint32_t lane,
+                                             uint32_t step) {
+    uint32_t c = 0;
+    if (lo >= hi) return 0;
+    for (uint32_t w = (lo >> 5) + lane; w <= (hi - 1) >> 5; w += step) {
+        uint32_t x = bits[w];
+        if (w == lo >> 5) x &= ~0u << (lo & 31);
+        if (w == (hi - 1) >> 5) x &= ~0u >> (31 - ((hi - 1) & 31));
+        c += __popc(x);
+    }
+    return c;
+}
+__device__ inline uint32_t abs_count_warp(const Absorbed &ab, uint32_t a, uint32_t f) {
+    const uint32_t lane = threadIdx.x & 31, lo = a + 1, hi = a + f + 1;
+    const uint32_t b0 = (lo + ab.W - 1) / ab.W, b1 = hi / ab.W;
+    uint32_t c = 0;
+    if (b0 < b1) {
+        for (uint32_t b = b0 + lane; b < b1; b += 32) c += ab.bwin[b];
+        c += abs_bits(ab.bits, lo, b0 * ab.W, lane, 32) + abs_bits(ab.bits, b1 * ab.W, hi, lane, 32);
+    } else {
+        c = abs_bits(ab.bits, lo, hi, lane, 32);
+    }
+    return __reduce_add_sync(0xffffffffu, c);
 }
 
 // Keep the candidates not inside a larger executed window; sort them into
@@ -744,7 +783,8 @@ __device__ __forceinline__ void k_plan_max_body(const Window *__restrict__ cand,
                                                   Window *small, Window *big, const UpdList u, uint8_t *pend,
                                                   DevStatus *st, uint32_t bid_, uint32_t nblk_,
                                                   uint32_t cut_group = CUT_GROUP_DEFAULT,
-                                                  uint32_t cut_shared = SMALL_WIN_SEGS) {
+                                                  uint32_t cut_shared = SMALL_WIN_SEGS,
+                                                  Absorbed ab = Absorbed{nullptr, nullptr, 0}) {
     // updates of segments that no window absorbed stay pending (overflow):
     // each update copies the mark its run's first update (the planner's
     // leader) wrote.  The marks are read only on the overflow paths that keep
@@ -779,6 +819,16 @@ __device__ __forceinline__ void k_plan_max_body(const Window *__restrict__ cand,
             hit |= (bitmap[bit >> 5] >> (bit & 31)) & 1u;
         }
         if (hit) cls = 4;
+    }
+    if (ab.bits) {  // uniform over the grid
+        uint32_t hid = (cls == 1 || cls == 2) ? abs_bits(ab.bits, w.a + 1, w.a + w.f + 1, 0, 1) : 0u;
+        for (uint32_t big = __ballot_sync(0xffffffffu, cls == 3); big; big &= big - 1) {
+            const int src = __ffs(big) - 1;
+            const uint32_t h = abs_count_warp(ab, __shfl_sync(0xffffffffu, w.a, src), __shfl_sync(0xffffffffu, w.f, src));
+            if ((int)(threadIdx.x & 31) == src) hid = h;
+        }
+        hid = __reduce_add_sync(0xffffffffu, hid);
+        if ((threadIdx.x & 31) == 0 && hid) atomicAdd(&st->abs_hidden, hid);
     }
     // the four classes' positions in one scan: a 16-bit field each (at most
     // TPB per block), classes 0 and 1 in the low word, 2 and 3 in the high
@@ -825,10 +875,15 @@ __global__ void __launch_bounds__(TPB) k_plan_max(const Window *__restrict__ can
                                                   const uint32_t *__restrict__ bitmap, Window *single, Window *small4,
                                                   Window *small, Window *big, const UpdList u, uint8_t *pend,
                                                   DevStatus *st, uint32_t cut_group, uint32_t cut_shared,
-                                                  DevStatus *pub) {
+                                                  DevStatus *pub, Absorbed ab) {
     griddep_wait();
-    k_plan_max_body(cand, n_cap, H, bitmap, single, small4, small, big, u, pend, st, blockIdx.x, gridDim.x, cut_group,
-                    cut_shared);
+    const uint32_t lim = st->ovf == 1u ? max(st->n_u, st->n_cand) : st->n_cand;
+    uint32_t c = blockIdx.x;
+    do {
+        k_plan_max_body(cand, n_cap, H, bitmap, single, small4, small, big, u, pend, st, c, gridDim.x, cut_group,
+                        cut_shared, ab);
+        c += gridDim.x;
+    } while ((uint64_t)c * TPB < lim);
     if (pub == nullptr) return;  // uniform over the grid
     __shared__ uint32_t last;
     __threadfence();  // this CTA's status atomics before its count
@@ -2017,14 +2072,19 @@ void launch_compact_pending(const UpdList in, const uint8_t *pend, uint32_t n, U
 void launch_plan(const UpdList u, uint32_t n_cap, const uint8_t *cnt, const uint32_t *P, int use_P,
                  uint64_t total_live, const unsigned long long *total_live_dev, uint32_t H, const Tables &tb,
                  uint32_t *bitmap, Window *cand, Window *single, Window *small4, Window *small, Window *big,
-                 uint8_t *pend, DevStatus *st, cudaStream_t s, DevStatus *pub) {
+                 uint8_t *pend, DevStatus *st, cudaStream_t s, DevStatus *pub, const BucketArgs *part) {
     ProfScope ps_("plan", s);
-    const uint32_t nb = (n_cap + TPB - 1) / TPB;
+    uint32_t nb = (n_cap + TPB - 1) / TPB;
     if (!nb) return;
+    Absorbed ab{nullptr, nullptr, 0};
+    if (part) {
+        nb = std::min<uint32_t>(nb, 152 * 4);
+        ab = Absorbed{part->absbits, part->bwin, 2u << (H - part->L)};
+    }
     launch_pdl(k_plan, dim3(nb), dim3(TPB), 0, s, u, n_cap, cnt, P, use_P, total_live, total_live_dev, H, tb, bitmap,
                cand, pend, st);
     launch_pdl(k_plan_max, dim3(nb), dim3(TPB), 0, s, cand, n_cap, H, bitmap, single, small4, small, big, u, pend, st,
-               tb.cut_group ? tb.cut_group : CUT_GROUP_DEFAULT, tb.cut_shared ? tb.cut_shared : SMALL_WIN_SEGS, pub);
+               tb.cut_group ? tb.cut_group : CUT_GROUP_DEFAULT, tb.cut_shared ? tb.cut_shared : SMALL_WIN_SEGS, pub, ab);
     note_launch(2);
 }
 
