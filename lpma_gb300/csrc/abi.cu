@@ -529,11 +529,43 @@ lpma_status_t tile_prep(LpmaHandle *h, const UpdList &u, uint32_t n_list, bool t
     return LPMA_OK;
 }
 
-// Execute the planned maximal windows (status already synced).
+// Whether the whole tree is spread anew in one pass: up to two updates a
+// segment, which the lanes that hold the segment merge.  1M segments with
+// 0.9 updates each took 177 us (gather and spread with their preparation:
+// 258), 32K segments with 0.5 each 39 (61), or 59 where the updates crowd
+// into a fiftieth of them (61).  Above, gather and spread give every update a
+// thread: a bulk load of 16.8M keys into 256K segments took them 200 us, the
+// one pass 890.
+bool respread_fits(const LpmaHandle *h, uint32_t n_list) {
+    return std::min(n_list, h->hst->n_u) <= 2 * nseg_of(h->H);
+}
+
+// Everything in the tree and the list's updates, m items, over tree dst.
+lpma_status_t respread(LpmaHandle *h, const UpdList &u, uint32_t n_list, uint64_t m, uint32_t thres, bool thres_active,
+                       Geo dst, uint8_t *cnt_d, ulonglong2 *fl_d, cudaStream_t s) {
+    if (m > nslots_of(dst.H)) return LPMA_ERR_INTERNAL;
+    launch_respread(Geo{h->c.keys, h->c.vals, h->H}, thres_active ? h->c.cnt_live : h->c.cnt, h->c.PQ, h->c.US, h->c.qi,
+                    h->c.done, u, n_list, thres_active ? thres : 0, thres_active, dst, (uint32_t)m, cnt_d, fl_d, h->sent,
+                    h->V, h->dst, s);
+    CK(cudaGetLastError());
+    return LPMA_OK;
+}
+// The same into the alternate slots and counts, which become the current ones.
+lpma_status_t respread_in_place(LpmaHandle *h, uint32_t hh, const UpdList &u, uint32_t n_list, uint64_t m,
+                                uint32_t thres, bool thres_active, cudaStream_t s) {
+    CKS(respread(h, u, n_list, m, thres, thres_active, Geo{h->c.keys_alt, h->c.vals_alt, hh}, h->c.cnt_alt, h->c.fl, s));
+    std::swap(h->c.keys, h->c.keys_alt);
+    std::swap(h->c.vals, h->c.vals_alt);
+    std::swap(h->c.cnt, h->c.cnt_alt);
+    return LPMA_OK;
+}
+
+// Execute the planned maximal windows (status already synced); live: the
+// items once they are.
 // small_done: the single / 4 / 32-segment windows were already launched
 // (the shared executors of a batched update).
-lpma_status_t exec_plan(LpmaHandle *h, const UpdList &u, uint32_t n_list, uint32_t thres, bool thres_active,
-                        cudaStream_t s, LpmaStats *st, bool small_done = false) {
+lpma_status_t exec_plan(LpmaHandle *h, const UpdList &u, uint32_t n_list, uint64_t live, uint32_t thres,
+                        bool thres_active, cudaStream_t s, LpmaStats *st, bool small_done = false) {
     const uint32_t n_single = h->hst->n_single, n_small4 = h->hst->n_small4, n_small = h->hst->n_small,
                    n_big = h->hst->n_big;
     Geo g{h->c.keys, h->c.vals, h->H};
@@ -549,7 +581,11 @@ lpma_status_t exec_plan(LpmaHandle *h, const UpdList &u, uint32_t n_list, uint32
     st->windows_small += n_single + n_small4 + n_small + n_abs;
     st->slots_rewritten += h->hst->slots_small + 32 * n_abs;
     st->slots_small += h->hst->slots_small + 32 * n_abs;
-    if (n_big) {
+    if (n_big == 1 && h->hst->root && respread_fits(h, n_list)) {  // the root window
+        CKS(respread_in_place(h, h->H, u, n_list, live, thres, thres_active, s));
+        st->windows_big += 1;
+        st->slots_rewritten += h->hst->slots_big;
+    } else if (n_big) {
         // the job list is built on the device (windows sorted by position,
         // tile prefix); the tile count came with the status read-back, so
         // the big windows need no host round trip
@@ -587,34 +623,41 @@ lpma_status_t level_up(LpmaHandle *h, cudaStream_t s) {
     return LPMA_OK;
 }
 
+// The whole tree and the list's updates over a tree of height hh (of the new
+// capacity, if there is one): gathered into the alternate slots, then spread.
+lpma_status_t gather_spread(LpmaHandle *h, uint32_t hh, const UpdList &u, uint32_t n_list, uint64_t m, uint32_t thres,
+                            bool thres_active, const Cap *fresh, cudaStream_t s) {
+    CKS(tile_prep(h, u, n_list, thres_active, s));
+    const Cap &c = fresh ? *fresh : h->c;
+    const uint32_t sf = (uint32_t)nseg_of(h->H), df = (uint32_t)nseg_of(hh);
+    if (!h->jobs_d) {
+        CK(dalloc(&h->jobs_d, 64));
+        h->jobs_cap = 64;
+    }
+    launch_set_job(h->jobs_d, TileJob{0, sf, 0, df, (uint32_t)m, 0, 0, 0}, s);
+    launch_exec_big(h->jobs_d, 1, (sf + 31) / 32, (df + 31) / 32, Geo{h->c.keys, h->c.vals, h->H}, h->c.PQ, h->c.US, u,
+                    n_list, thres_active ? thres : 0, c.keys_alt, c.vals_alt, nslots_of(c.Hc), Geo{c.keys, c.vals, hh},
+                    c.cnt, c.fl, h->sent, h->V, h->dst, s);
+    CK(cudaGetLastError());
+    return LPMA_OK;
+}
+
 // Rebuild at height hh (rebuild_rpma, rpma.cuh:1417-1472): every kept key of
 // the current array plus the list's inserts, spread over the new array.
 lpma_status_t rebuild(LpmaHandle *h, uint32_t hh, const UpdList &u, uint32_t n_list, uint64_t m, uint32_t thres,
                       bool thres_active, cudaStream_t s, LpmaStats *st) {
     if (hh > LPMA_MAX_HEIGHT) return LPMA_ERR_CAPACITY;
     const uint32_t H = h->H;
-    CKS(tile_prep(h, u, n_list, thres_active, s));
+    const bool fused = respread_fits(h, n_list);
     Cap fresh;
     const bool grow = hh > h->c.Hc;
     if (grow) CK(alloc_cap(fresh, std::min<uint32_t>(hh + 1, LPMA_MAX_HEIGHT), s));
-    // gather into the alternate buffer, spread into the main buffer (of the
-    // new capacity when the tree outgrows the current one)
-    Geo src{h->c.keys, h->c.vals, H};
-    Geo dst = grow ? Geo{fresh.keys, fresh.vals, hh} : Geo{h->c.keys, h->c.vals, hh};
-    uint64_t *Mk = grow ? fresh.keys_alt : h->c.keys_alt;
-    uint8_t *Mv = grow ? fresh.vals_alt : h->c.vals_alt;
-    uint8_t *cnt_d = grow ? fresh.cnt : h->c.cnt;
-    ulonglong2 *fl_d = grow ? fresh.fl : h->c.fl;
-    const uint32_t sf = (uint32_t)nseg_of(H), df = (uint32_t)nseg_of(hh);
-    if (!h->jobs_d) {
-        CK(dalloc(&h->jobs_d, 64));
-        h->jobs_cap = 64;
-    }
-    launch_set_job(h->jobs_d, TileJob{0, sf, 0, df, (uint32_t)m, 0, 0, 0}, s);
-    const uint64_t m_cap = nslots_of(grow ? fresh.Hc : h->c.Hc);
-    launch_exec_big(h->jobs_d, 1, (sf + 31) / 32, (df + 31) / 32, src, h->c.PQ, h->c.US, u, n_list,
-                    thres_active ? thres : 0, Mk, Mv, m_cap, dst, cnt_d, fl_d, h->sent, h->V, h->dst, s);
-    CK(cudaGetLastError());
+    if (fused && grow)
+        CKS(respread(h, u, n_list, m, thres, thres_active, Geo{fresh.keys, fresh.vals, hh}, fresh.cnt, fresh.fl, s));
+    else if (fused)
+        CKS(respread_in_place(h, hh, u, n_list, m, thres, thres_active, s));
+    else
+        CKS(gather_spread(h, hh, u, n_list, m, thres, thres_active, grow ? &fresh : nullptr, s));
     if (grow) {
         free_cap(h->c, s);  // in stream order, after the gather read it
         h->c = fresh;
@@ -985,7 +1028,7 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
     lpma_status_t r = LPMA_OK;
     if (n_new + n_gone > 0 && !h->hst->ovf) {
         const bool root = h->hst->root != 0;
-        r = exec_plan(h, h->u, (uint32_t)n, thres, thres_active, s, &st, small_done);
+        r = exec_plan(h, h->u, (uint32_t)n, (uint64_t)live_after, thres, thres_active, s, &st, small_done);
         if (r == LPMA_OK && root) {
             st.root_executed = 1;
             st.levelup = 1;  // update_rpma returns true once the root absorbed (rpma.cuh:1646-1653)
@@ -1000,7 +1043,7 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
         const uint32_t hh = min_height((uint64_t)live_after);
         if (hh == h->H + 1) {
             st.levelup_path = 1;
-            r = exec_plan(h, h->u, (uint32_t)n, thres, thres_active, s, &st);
+            r = exec_plan(h, h->u, (uint32_t)n, (uint64_t)live_after, thres, thres_active, s, &st);
             if (r == LPMA_OK) r = level_up(h, s);
             if (r == LPMA_OK) {
                 launch_compact_pending(h->u, h->pend, n_u, h->u2, h->blk_nn, h->blk_ins, h->dst, s);
@@ -1024,7 +1067,7 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
                     r = rebuild(h, min_height((uint64_t)live_after), h->u2, n2, (uint64_t)live_after, thres,
                                 thres_active, s, &st);
                 } else if (r == LPMA_OK) {
-                    r = exec_plan(h, h->u2, n2, thres, thres_active, s, &st);
+                    r = exec_plan(h, h->u2, n2, (uint64_t)live_after, thres, thres_active, s, &st);
                     if (r == LPMA_OK && h->H > 0) {  // fill_empty_segs, rpma.cuh:1474-1530
                         CK(cudaMemsetAsync(&h->dst->empty_found, 0, 4, s));
                         launch_check_empty_level(h->c.cnt, h->H, h->dst, s);

@@ -169,6 +169,15 @@ void launch_exec_big(const TileJob *jobs, uint32_t njobs, uint32_t stiles, uint3
                      uint64_t *Mk, uint8_t *Mv, uint64_t m_cap, Geo dst, uint8_t *cnt_d, ulonglong2 *fl_d,
                      uint32_t *sent, uint32_t V, DevStatus *st, cudaStream_t s);
 
+// All items of src (counts cnt, the live ones with an active expiry threshold
+// th) and the list's updates, m items (<= dst's slots), spread evenly over
+// dst, which has other slots than src; cnt_d is not cnt.  part and ustart
+// hold a word per 32 source segments and one more, base one per 16,384;
+// done as for the view.
+void launch_respread(Geo src, const uint8_t *cnt, uint32_t *part, uint32_t *ustart, uint32_t *base, uint32_t *done,
+                     const UpdList u, uint32_t n_cap, uint32_t thres, bool th, Geo dst, uint32_t m, uint8_t *cnt_d,
+                     ulonglong2 *fl_d, uint32_t *sent, uint32_t V, DevStatus *st, cudaStream_t s);
+
 // The big windows (n, count known on the host) as tile jobs in order of
 // their first segment, built on the device: the window list is sorted by
 // position in the scratch arrays, then one CTA scans the tile counts.

@@ -1979,6 +1979,400 @@ __global__ void __launch_bounds__(GT_TPB) k_spread(const TileJob *__restrict__ j
     }
 }
 
+// ------------------------------------------------------------------ respread
+// The whole array (a root window, or a rebuild at another height) goes from
+// one slot array to another in one pass.  A CTA takes 128 destination
+// segments, so at most 4,096 ranks, finds the source segments that hold
+// them, merges their kept slots and inserts in shared memory in rank order
+// and writes its segments whole.
+//
+// It reads the occupied slots once and writes all slots once; gather and
+// spread write and read a contiguous copy in between, after counts per
+// segment, a scan of them and a sorted job list.  Bound by instructions (the
+// merge of four segments a warp takes about 350; half of the issue slots)
+// and the chain of dependent reads from the rank to the slots; HBM is at 30%.
+// 15.2M items and 1M updates over 1M segments: 165 us and 12 for the tiles'
+// prefixes (258 us before).  With 128 destination segments a CTA it took 240
+// (4 or 5 of the 8 warps had a tile), with 256 190 (a ninth tile).
+constexpr uint32_t RS_RANKS = 4096;  // items a CTA merges at most
+constexpr uint32_t RS_TILE = 32;    // source segments a warp takes at a time
+constexpr uint32_t RS_GROUP = 512;  // tiles under one base count
+constexpr uint32_t RS_LOCAL = 8;    // updates that a segment's lanes merge in a tile of more than 32
+constexpr uint32_t RS_BUSY = 256;   // segments with more that the CTA merges together
+
+// ustart[t]: tile t's first update.  part[t] + base[t / 512]: the items
+// before tile t once the updates before it are done, t = 0 .. ntiles.
+__global__ void __launch_bounds__(1024) k_rs_tiles(const uint8_t *__restrict__ cnt, uint64_t nseg, uint32_t ntiles,
+                                                   const UpdList u, uint32_t n_cap, const DevStatus *st, uint32_t *part,
+                                                   uint32_t *ustart, uint32_t *base, uint32_t *done) {
+    const uint32_t t = blockIdx.x * RS_GROUP + (threadIdx.x >> 1);  // 2 threads a tile
+    const uint64_t s0 = (uint64_t)t * RS_TILE + 16 * (threadIdx.x & 1);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t c = 0;
+    if (s0 + 16 <= nseg) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(cnt + s0);
+        c = __dp4a(v.x, 0x01010101u, c);
+        c = __dp4a(v.y, 0x01010101u, c);
+        c = __dp4a(v.z, 0x01010101u, c);
+        c = __dp4a(v.w, 0x01010101u, c);
+    } else {
+        for (uint64_t s = s0; s < nseg; s++) c += cnt[s];
+    }
+    __shared__ uint32_t last, ws[32];
+    uint32_t v = c;  // inclusive over the CTA's half tiles
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
+    }
+    if (lane == 31) ws[w] = v;
+    __syncthreads();
+    uint32_t total = 0;
+#pragma unroll
+    for (int k = 0; k < 32; k++) {
+        const uint32_t y = ws[k];
+        v += k < w ? y : 0u;
+        total += y;
+    }
+    if ((threadIdx.x & 1) == 0 && t <= ntiles) {
+        const uint32_t nu = min(st->n_u, n_cap);
+        uint32_t L = 0, R = nu;
+        while (L < R) {  // eight ways at once: a third of the dependent reads
+            const uint32_t step = (R - L + 7) >> 3;
+            uint32_t b = 0;
+#pragma unroll
+            for (uint32_t i = 1; i < 8; i++) {
+                const uint32_t p = L + i * step - 1;
+                b += (p < R && u.seg[p] < t * RS_TILE) ? 1u : 0u;
+            }
+            R = b == 7 ? R : min(R, L + (b + 1) * step - 1);
+            L += b * step;
+        }
+        if (t == ntiles) L = nu;
+        ustart[t] = L;
+        part[t] = v - c + (nu ? 2 * u.ip[L] - L : 0u);  // inserts less deletes before it
+    }
+    if (threadIdx.x == 0) base[blockIdx.x] = total;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1 ? 1u : 0u;  // 0 again for the next call
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    uint32_t carry = 0;  // the last CTA: base becomes its own exclusive scan
+    for (uint32_t b0 = 0; b0 < gridDim.x; b0 += 1024) {
+        const uint32_t i = b0 + threadIdx.x;
+        const uint32_t x = i < gridDim.x ? __ldcg(base + i) : 0u;
+        uint32_t s = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += y;
+        }
+        if (lane == 31) ws[w] = s;
+        __syncthreads();
+        uint32_t off = carry + s - x;
+#pragma unroll
+        for (int k = 0; k < 32; k++) {
+            const uint32_t y = ws[k];
+            off += k < w ? y : 0u;
+            carry += y;
+        }
+        if (i < gridDim.x) base[i] = off;
+        __syncthreads();
+    }
+}
+
+struct RsSmem {
+    uint64_t k[RS_RANKS];
+    uint8_t v[RS_RANKS];
+    uint32_t list[256];               // source tiles with items of this CTA's
+    uint32_t b_seg[RS_BUSY], b_us[RS_BUSY], b_ue[RS_BUSY], b_base[RS_BUSY];
+    uint32_t nlist, nbusy, group, tile;
+};
+
+// The inserts [first, last) of segment s by step from x0 on, into their ranks.
+template <bool TH, class Put>
+__device__ __forceinline__ void rs_busy(const Geo &src, const UpdList &u, uint32_t s, uint32_t us, uint32_t ue,
+                                        uint32_t base, uint32_t w0, uint32_t w1, uint32_t thres, uint32_t tid,
+                                        uint32_t step, Put put) {
+    // a rank is at most 32 above the inserts before it
+    const uint32_t ip0 = u.ip[us], lo = w0 > base + 32 ? w0 - base - 32 : 0u;
+    uint32_t L = us, R = ue;
+    while (lo && L < R) {
+        const uint32_t mid = (L + R) >> 1;
+        if (u.ip[mid] - ip0 < lo)
+            L = mid + 1;
+        else
+            R = mid;
+    }
+    const uint64_t j = heap_of_linear32(s, src.H);
+    const uint64_t *sk = src.keys + 32 * j;
+    const uint8_t *sv = src.vals + 32 * j;
+    for (uint32_t x = L + tid; x < ue; x += step) {
+        const uint32_t ri = u.ip[x] - ip0;
+        if (base + ri >= w1) break;
+        if (u.kind[x] != KIND_INS) continue;
+        const uint64_t y = u.key[x];
+        uint32_t pos = 0;  // slots below y (the segment is sorted, NONE-padded)
+#pragma unroll
+        for (uint32_t st = 16; st; st >>= 1)
+            if (sk[pos + st - 1] < y) pos += st;
+        if (sk[pos] < y) pos++;
+        // of which this batch deletes, or has expired
+        uint32_t gone = (x - us) - ri;
+        if (TH)
+            for (uint32_t z = 0; z < pos; z++)
+                gone += (sv[z] != VAL_TOMB && !kept_t<TH>(sk[z], sv[z], thres)) ? 1u : 0u;
+        put(base + ri + pos - gone, y, u.val[x]);
+    }
+}
+
+template <bool TH>
+__global__ void __launch_bounds__(256, 4) k_respread(Geo src, uint64_t nseg, const uint8_t *__restrict__ cnt,
+                                                     const uint32_t *__restrict__ part,
+                                                     const uint32_t *__restrict__ ustart,
+                                                     const uint32_t *__restrict__ base_of, const UpdList u,
+                                                     uint32_t thres, Geo dst, uint32_t df, uint32_t nd, uint32_t m, uint8_t *cnt_d,
+                                                     ulonglong2 *fl_d, uint32_t *sent, uint32_t V, DevStatus *st) {
+    __shared__ __align__(16) RsSmem S;
+    const uint32_t ntiles = (uint32_t)((nseg + RS_TILE - 1) / RS_TILE), ngroups = ntiles / RS_GROUP + 1;
+    const uint32_t tid = threadIdx.x;
+    const int lane = tid & 31, w = tid >> 5, gl = lane & 7, g = lane >> 3;
+    const uint32_t k0 = blockIdx.x * nd, k1 = min(df, k0 + nd);
+    const uint64_t inv = ~0ull / df;
+    const uint32_t F0 = (uint32_t)first_rank_recip(k0, m, df, inv), F1 = (uint32_t)first_rank_recip(k1, m, df, inv);
+    auto items_before = [&](uint32_t t) { return part[t] + base_of[t / RS_GROUP]; };
+    const uint32_t nr = F1 - F0;
+    auto put = [&](uint32_t r, uint64_t key, uint8_t val) {
+        const uint32_t i = r - F0;
+        if (i < nr) {
+            S.k[i] = key;
+            S.v[i] = val;
+        }
+    };
+    if (k1 == df) {
+        if (tid < 64) cnt_d[df + tid] = 0;  // the counts' padding
+        if (tid == 0 && items_before(ntiles) != m) {  // every item accounted for
+            atomicOr(&st->sticky, ERR_INTERNAL);
+            atomicCAS(&st->sticky_site, 0u, 2u);
+        }
+    }
+    if (F1 > F0) {
+        // the tile of the first item: the last one with no more than F0 before it
+        if (tid == 0) S.group = S.tile = S.nlist = S.nbusy = 0;
+        __syncthreads();
+        for (uint32_t b = tid; b < ngroups; b += 256)
+            if (b * RS_GROUP <= ntiles && items_before(b * RS_GROUP) <= F0) atomicMax(&S.group, b);
+        __syncthreads();
+        {
+            const uint32_t t0 = S.group * RS_GROUP;
+            for (uint32_t t = t0 + tid; t < min(t0 + RS_GROUP, ntiles); t += 256)
+                if (items_before(t) <= F0) atomicMax(&S.tile, t);
+        }
+        __syncthreads();
+        for (uint32_t tb = S.tile;; tb += 256) {
+            if (tb + tid < ntiles) {
+                const uint32_t a = items_before(tb + tid), b = items_before(tb + tid + 1);
+                if (b > a && b > F0 && a < F1) S.list[atomicAdd(&S.nlist, 1u)] = tb + tid;
+            }
+            __syncthreads();
+            const uint32_t nl = S.nlist;
+            for (uint32_t q = w; q < nl; q += 8) {  // a warp a tile
+                const uint32_t t = S.list[q], s = t * RS_TILE + lane;
+                const uint32_t U0 = ustart[t], U1 = ustart[t + 1], n_upd = U1 - U0;
+                const uint32_t T0 = items_before(t), T1 = items_before(t + 1);
+                const uint32_t c = s < nseg ? cnt[s] : 0u;
+                // the tile's updates in registers, a lane each, if they fit
+                const bool few = n_upd <= 32;
+                uint32_t ysv = 0xFFFFFFFFu;
+                uint64_t yk = KEY_NONE;
+                bool yins = false;
+                uint8_t yv = 0;
+                if (few && (uint32_t)lane < n_upd) {
+                    const uint32_t x = U0 + lane;
+                    ysv = u.seg[x];
+                    yk = u.key[x];
+                    yins = u.kind[x] == KIND_INS;
+                    yv = u.val[x];
+                }
+                const uint32_t insm = __ballot_sync(0xffffffffu, yins);
+                uint32_t us = U0, pi;  // the lane's segment's first update, the tile's inserts before it
+                if (few) {
+                    uint32_t pos = 0;
+#pragma unroll
+                    for (uint32_t step = 16; step; step >>= 1) {
+                        const uint32_t y = __shfl_sync(0xffffffffu, ysv, pos + step - 1);
+                        if (y < s) pos += step;
+                    }
+                    if (__shfl_sync(0xffffffffu, ysv, pos) < s) pos++;
+                    us += pos;
+                    pi = __popc(insm & (uint32_t)((1ull << pos) - 1));
+                } else {
+                    uint32_t R = U1;
+                    while (us < R) {
+                        const uint32_t mid = (us + R) >> 1;
+                        if (u.seg[mid] < s)
+                            us = mid + 1;
+                        else
+                            R = mid;
+                    }
+                    pi = u.ip[us];
+                    pi -= __shfl_sync(0xffffffffu, pi, 0);
+                }
+                uint32_t incl = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                const uint32_t base = T0 + incl - c + 2 * pi - (us - U0);
+                uint32_t ue = __shfl_down_sync(0xffffffffu, us, 1), end = __shfl_down_sync(0xffffffffu, base, 1);
+                if (lane == 31) ue = U1, end = T1;
+                const bool mine = s < nseg && end > base && end > F0 && base < F1;
+                uint32_t alone = 0;  // busy segments that the list has no room for
+                if (mine && !few && ue - us > RS_LOCAL) {
+                    const uint32_t at = atomicAdd(&S.nbusy, 1u);
+                    if (at < RS_BUSY) {
+                        S.b_seg[at] = s;
+                        S.b_us[at] = us;
+                        S.b_ue[at] = ue;
+                        S.b_base[at] = base;
+                    } else {
+                        alone = 1;
+                    }
+                }
+                const uint32_t act = __ballot_sync(0xffffffffu, mine);
+                alone = __ballot_sync(0xffffffffu, alone != 0);
+                uint64_t k[2][4];
+                uint32_t v4[2];
+                auto load = [&](uint32_t it, int b) {
+                    const uint32_t i = 4 * it + g;
+                    // without expiry, c slots of the segment are taken
+                    const uint32_t ci = TH ? 32u : __shfl_sync(0xffffffffu, c, i);
+                    k[b][0] = k[b][1] = k[b][2] = k[b][3] = KEY_NONE;
+                    v4[b] = 0;
+                    if (((act >> i) & 1u) && 4u * gl < ci) {
+                        const uint64_t j = heap_of_linear32(t * RS_TILE + i, src.H);
+                        const ulonglong2 *kp = reinterpret_cast<const ulonglong2 *>(src.keys + 32 * j + 4 * gl);
+                        const ulonglong2 x = kp[0], y = kp[1];
+                        v4[b] = *reinterpret_cast<const uint32_t *>(src.vals + 32 * j + 4 * gl);
+                        k[b][0] = x.x, k[b][1] = x.y, k[b][2] = y.x, k[b][3] = y.y;
+                    }
+                };
+                load(0, 0);
+#pragma unroll 2
+                for (uint32_t it = 0; it < 8; it++) {
+                    const int b = it & 1;
+                    if (it + 1 < 8) load(it + 1, b ^ 1);
+                    const uint32_t i = 4 * it + g;
+                    const bool active = (act >> i) & 1u;
+                    const uint32_t b_us = __shfl_sync(0xffffffffu, us, i), b_ue = __shfl_sync(0xffffffffu, ue, i);
+                    const uint32_t b_base = __shfl_sync(0xffffffffu, base, i);
+                    const uint32_t nupd = active ? b_ue - b_us : 0u;
+                    uint32_t kmask = 0;
+#pragma unroll
+                    for (int z = 0; z < 4; z++)
+                        if (active && kept_t<TH>(k[b][z], (uint8_t)(v4[b] >> (8 * z)), thres)) kmask |= 1u << z;
+                    const uint32_t kept = __popc(kmask);
+                    uint32_t ki = kept;
+#pragma unroll
+                    for (int o = 1; o < 8; o <<= 1) {
+                        const uint32_t y = __shfl_up_sync(0xffffffffu, ki, o, 8);
+                        if (gl >= o) ki += y;
+                    }
+                    ki -= kept;
+                    // The segment's inserts (a bit each), one after the other:
+                    // the lane whose slots it falls into or behind puts it.
+                    const bool local = few || nupd <= RS_LOCAL;
+                    uint64_t uk = yk;
+                    uint32_t uv = yv, from = b_us - U0, im = 0;
+                    if (few) {
+                        im = nupd ? (insm >> from) & (0xFFFFFFFFu >> (32 - nupd)) : 0u;
+                    } else {
+                        const bool has = local && (uint32_t)gl < nupd;
+                        uk = has ? u.key[b_us + gl] : KEY_NONE;
+                        uv = has ? u.val[b_us + gl] : 0u;
+                        im = (__ballot_sync(0xffffffffu, has && u.kind[b_us + gl] == KIND_INS) >> (lane & 24)) & 0xffu;
+                        from = lane & 24;
+                    }
+                    uint32_t below[4] = {0, 0, 0, 0};
+                    for (uint32_t r = 0; __any_sync(0xffffffffu, im != 0); r++) {
+                        const uint32_t src_lane = (from + __ffs(im) - 1) & 31;
+                        const uint64_t y = __shfl_sync(0xffffffffu, uk, src_lane);
+                        const uint32_t yval = __shfl_sync(0xffffffffu, uv, src_lane);
+                        const bool on = im != 0;
+                        uint32_t less = 0;
+#pragma unroll
+                        for (int z = 0; z < 4; z++) {
+                            const bool p = k[b][z] < y;
+                            less |= p ? 1u << z : 0u;
+                            below[z] += (on && !p) ? 1u : 0u;
+                        }
+                        const uint32_t nb = __popc((__ballot_sync(0xffffffffu, less & 1u) >> (lane & 24)) & 0xffu);
+                        if (on && (nb ? nb - 1 : 0u) == (uint32_t)gl)
+                            put(b_base + r + ki + __popc(kmask & less), y, (uint8_t)yval);
+                        im &= im - 1;
+                    }
+#pragma unroll
+                    for (int z = 0; z < 4; z++)
+                        if ((kmask >> z) & 1u) {
+                            const uint32_t bl =
+                                local ? below[z] : u.ip[lb_key(u.key, b_us, b_ue, k[b][z])] - u.ip[b_us];
+                            put(b_base + ki + __popc(kmask & ((1u << z) - 1)) + bl, k[b][z],
+                                (uint8_t)(v4[b] >> (8 * z)));
+                        }
+                }
+                for (; alone; alone &= alone - 1) {
+                    const int i = __ffs(alone) - 1;
+                    rs_busy<TH>(src, u, t * RS_TILE + i, __shfl_sync(0xffffffffu, us, i), __shfl_sync(0xffffffffu, ue, i),
+                                __shfl_sync(0xffffffffu, base, i), F0, F1, thres, lane, 32, put);
+                }
+            }
+            __syncthreads();
+            const uint32_t nb = min(S.nbusy, RS_BUSY);
+            for (uint32_t q = w; q < nb; q += 8)  // a warp each, and the CTA together where it is a chain
+                if (S.b_ue[q] - S.b_us[q] <= 256)
+                    rs_busy<TH>(src, u, S.b_seg[q], S.b_us[q], S.b_ue[q], S.b_base[q], F0, F1, thres, lane, 32, put);
+            for (uint32_t q = 0; q < nb; q++)
+                if (S.b_ue[q] - S.b_us[q] > 256)
+                    rs_busy<TH>(src, u, S.b_seg[q], S.b_us[q], S.b_ue[q], S.b_base[q], F0, F1, thres, tid, 256, put);
+            const bool more = tb + 256 < ntiles && items_before(tb + 256) < F1;  // the same in every thread
+            __syncthreads();
+            if (!more) break;
+            if (tid == 0) S.nlist = S.nbusy = 0;
+            __syncthreads();
+        }
+    }
+    for (uint32_t k = k0 + (tid >> 3); k < k1; k += 32) {
+        const uint32_t f0 = (uint32_t)first_rank_recip(k, m, df, inv), nk = (uint32_t)first_rank_recip(k + 1, m, df, inv) - f0;
+        const uint64_t j = heap_of_linear32(k, dst.H);
+        uint64_t o[4];
+        uint32_t ov = 0;
+#pragma unroll
+        for (int z = 0; z < 4; z++) {
+            const uint32_t slot = 4 * gl + z, r = f0 + slot - F0;
+            o[z] = KEY_NONE;
+            if (slot < nk) {
+                o[z] = S.k[r];
+                ov |= (uint32_t)S.v[r] << (8 * z);
+                if (is_sentinel(o[z])) {
+                    const uint32_t row = (uint32_t)(o[z] >> SRC_SHIFT);
+                    if (row < V) sent[row] = (uint32_t)(32 * j + slot);
+                }
+            }
+        }
+        ulonglong2 *kp = reinterpret_cast<ulonglong2 *>(dst.keys + 32 * j + 4 * gl);
+        kp[0] = make_ulonglong2(o[0], o[1]);
+        kp[1] = make_ulonglong2(o[2], o[3]);
+        *reinterpret_cast<uint32_t *>(dst.vals + 32 * j + 4 * gl) = ov;
+        if (gl == 0) {
+            fl_d[j] = nk ? make_ulonglong2(S.k[f0 - F0], S.k[f0 + nk - 1 - F0]) : make_ulonglong2(KEY_NONE, KEY_NONE);
+            cnt_d[k] = (uint8_t)nk;
+        }
+    }
+}
+
 // ------------------------------------------------------------------ levels
 __global__ void __launch_bounds__(TPB) k_levelup_cnt(const uint8_t *__restrict__ cnt_old, uint8_t *cnt_new,
                                                      uint32_t H_old) {
@@ -2160,6 +2554,27 @@ void launch_exec_big(const TileJob *jobs, uint32_t njobs, uint32_t stiles, uint3
                                                                  fl_d, sent, V, st);
     }
     note_launch(n_upd ? 3 : 2);
+}
+
+void launch_respread(Geo src, const uint8_t *cnt, uint32_t *part, uint32_t *ustart, uint32_t *base, uint32_t *done,
+                     const UpdList u, uint32_t n_cap, uint32_t thres, bool th, Geo dst, uint32_t m, uint8_t *cnt_d,
+                     ulonglong2 *fl_d, uint32_t *sent, uint32_t V, DevStatus *st, cudaStream_t s) {
+    const uint64_t nseg = nseg_of(src.H);
+    const uint32_t ntiles = (uint32_t)((nseg + RS_TILE - 1) / RS_TILE), df = (uint32_t)nseg_of(dst.H);
+    {
+        ProfScope ps_("respread_tiles", s);
+        k_rs_tiles<<<ntiles / RS_GROUP + 1, 2 * RS_GROUP, 0, s>>>(cnt, nseg, ntiles, u, n_cap, st, part, ustart, base, done);
+    }
+    ProfScope ps_("respread", s);
+    // As many destination segments a CTA as its ranks allow (a segment takes
+    // ceil(m / df) items at most) and as come from 7 source tiles on average,
+    // mostly 8, a warp each; fewer where the CTAs would not fill the chip.
+    const uint32_t most = RS_RANKS / std::max<uint32_t>(1, (uint32_t)(((uint64_t)m + df - 1) / df));
+    const uint32_t even = (uint32_t)std::max<uint64_t>(32, 7ull * RS_TILE * df / nseg);
+    const uint32_t nd = std::min({1024u, most, even, std::max(32u, df / (152 * 4))});
+    (th ? k_respread<true> : k_respread<false>)<<<(df + nd - 1) / nd, 256, 0, s>>>(
+        src, nseg, cnt, part, ustart, base, u, thres, dst, df, nd, m, cnt_d, fl_d, sent, V, st);
+    note_launch(2);
 }
 
 namespace {
