@@ -176,10 +176,6 @@ bool pagerank_pulls(uint64_t edges, uint32_t iterations) {
     return iterations >= 3 && edges >= (1u << 17) && edges * iterations >= (3u << 20);
 }
 
-// calls on the sorted front after a batch whose buckets overflowed: a stream
-// of such batches pays the vain partition (about 30 us) once in 17 calls
-constexpr uint32_t PART_SKIP = 16;
-
 // levels of a BFS launched before the host reads their counters back, the
 // counters of those levels (ranges and vertices of each frontier), and the
 // words of the read paths' pinned buffer

@@ -46,6 +46,9 @@ const void *pack_kernel_fn();
 // ordered, resolved and single-segment windows executed bucket by bucket
 constexpr uint32_t PART_L_MAX = 11, PART_IPT = 8;
 constexpr uint64_t PART_MIN = 256, PART_MAX = 1u << 21;  // keys of a batch
+// calls on the sorted front after a batch whose buckets overflowed: a stream
+// of such batches pays the vain partition (about 30 us) once in 17 calls
+constexpr uint32_t PART_SKIP = 16;
 struct PartPlan {
     uint32_t L;    // 2^L buckets; 0: the sorted front takes the batch
     uint32_t cap;  // entries of a bucket
