@@ -754,7 +754,8 @@ lpma_status_t enqueue_part(LpmaHandle *h, cudaStream_t s, const PartArgs &pa, si
     const Geo g{h->c.keys, h->c.vals, h->H};
     const BucketArgs ba{g, h->c.fl, h->c.cnt, thres_active ? h->c.cnt_live : nullptr, h->sent, h->V, pa.thres,
                         tb.lower[0], pp.L, pp.cap, h->part_ent, pa.fill, pa.fill + (1u << PART_L_MAX),
-                        pa.fill + (2u << PART_L_MAX), h->c.absbits, h->dst};
+                        pa.fill + (2u << PART_L_MAX), h->c.absbits, h->c.bitmap, (uint32_t)bitmap_words(h->H),
+                        pp.stage, h->dst};
     launch_buckets(ba, h->u, s);
     const bool pub = front_publishes(h);
     CKS(run_plan(h, h->u, (uint32_t)n, thres_active, 0, tb, s,
@@ -783,7 +784,7 @@ lpma_status_t enqueue_part(LpmaHandle *h, cudaStream_t s, const PartArgs &pa, si
 // for the engine's own sentinels, a sort tier set by the caller, or a handle
 // whose buckets overflowed lately.
 PartPlan plan_part(LpmaHandle *h, size_t n, bool internal) {
-    if (internal || h->part_skip || sort_tier_forced((uint32_t)n, h->sort)) return PartPlan{0, 0, 0};
+    if (internal || h->part_skip || sort_tier_forced((uint32_t)n, h->sort)) return PartPlan{};
     return part_plan(n, h->H);
 }
 
@@ -834,7 +835,7 @@ lpma_status_t run_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, cons
     h->front_part = pp.L != 0;
     if (pp.L) CKS(ensure_part(h, pp, s));
     const PartArgs pa{ins, ins_vals, del, (uint32_t)n_ins, (uint32_t)n_del, h->V, thres, h->cfg.key_format, pp.L, pp.cap,
-                      pp.ipt, h->c.fl, h->part_ent, h->part_ctl, h->c.bitmap, (uint32_t)bitmap_words(h->H), h->dst};
+                      pp.ipt, h->c.fl, h->part_ent, h->part_ctl, h->dst};
     auto enqueue = [&](cudaStream_t st) {
         return pp.L ? enqueue_part(h, st, pa, n, pp, thres_active)
                     : enqueue_front(h, st, ins, ins_vals, n_ins, del, n_del, thres, thres_active, internal);

@@ -59,8 +59,9 @@ __global__ void __launch_bounds__(PT) k_part(PartArgs a) {
     const uint32_t NB = 1u << a.L, ntop = NB - 1;
     uint64_t *first = reinterpret_cast<uint64_t *>(smem), *last = first + NB;  // the top nodes' bounds
     uint32_t *hist = reinterpret_cast<uint32_t *>(last + NB);
-    // the planner bitmap of this call starts clear
-    for (uint32_t i = blockIdx.x * PT + threadIdx.x; i < a.bitmap_words; i += gridDim.x * PT) a.bitmap[i] = 0;
+    const uint32_t n = a.n_ins + a.n_del, tile = a.ipt * PT, i0 = blockIdx.x * tile + threadIdx.x;
+    uint64_t key[PART_IPT];
+    uint32_t pay[PART_IPT], bkt[PART_IPT], at[PART_IPT];
     bool hole = false;
     for (uint32_t t = threadIdx.x; t < ntop; t += PT) {
         const ulonglong2 f = a.fl[t];
@@ -70,12 +71,7 @@ __global__ void __launch_bounds__(PT) k_part(PartArgs a) {
     }
     for (uint32_t t = threadIdx.x; t < NB; t += PT) hist[t] = 0;
     hole = __syncthreads_or(hole);
-    const uint32_t n = a.n_ins + a.n_del;
     uint32_t mint = 0xFFFFFFFFu, bad = 0xFFFFFFFFu;
-    const uint32_t tile = a.ipt * PT;
-    const uint32_t i0 = blockIdx.x * tile + threadIdx.x;
-    uint64_t key[PART_IPT];
-    uint32_t pay[PART_IPT], bkt[PART_IPT], at[PART_IPT];
 #pragma unroll
     for (uint32_t q = 0; q < PART_IPT; q++) {
         const uint32_t i = i0 + q * PT;
@@ -266,6 +262,17 @@ __global__ void __launch_bounds__(BT, BUCKET_CTAS) k_bucket(BucketArgs a) {
     uint16_t *sseg = reinterpret_cast<uint16_t *>(sc + a.cap), *el = sseg + a.cap;
     const uint32_t b = blockIdx.x, W = 2u << (a.g.H - a.L);
     const int lane = threadIdx.x & 31;
+    // Before the partition is done: the planner's bitmap of this call starts
+    // clear, and the top levels of the bucket's subtree come in.  Node (level
+    // l, position p) of bucket b's subtree is heap index
+    // 2^(L+l) - 1 + (b << l) + p.
+    const uint32_t h = a.g.H - a.L;  // its height
+    const uint32_t sl = a.stage ? staged_levels(h) : 0;
+    for (uint32_t i = b * BT + threadIdx.x; i < a.bitmap_words; i += gridDim.x * BT) a.bitmap[i] = 0;
+    for (uint32_t t = threadIdx.x; t + 1 < (1u << sl); t += BT) {
+        const uint32_t l = 31 - __clz(t + 1), p = t + 1 - (1u << l);
+        sub[t] = a.fl[((1u << (a.L + l)) - 1) + (b << l) + p];
+    }
     griddep_wait();
     // a rejected batch, or one whose buckets overflowed, changes nothing
     if (a.st->error | a.st->part_ovf) return;
@@ -279,18 +286,6 @@ __global__ void __launch_bounds__(BT, BUCKET_CTAS) k_bucket(BucketArgs a) {
         return;
     }
     const ulonglong2 *ent = a.ent + (uint64_t)b * a.cap;
-    // the subtree of bucket b: node (level l, position p) is heap index
-    // 2^(L+l) - 1 + (b << l) + p; its top levels are staged when the bucket
-    // has keys enough to pay for it
-    const uint32_t h = a.g.H - a.L;  // its height
-    uint32_t sl = 0;                 // staged levels
-    if (c >= 64) {
-        sl = staged_levels(h);
-        for (uint32_t t = threadIdx.x; t < (1u << sl) - 1; t += BT) {
-            const uint32_t l = 31 - __clz(t + 1), p = t + 1 - (1u << l);
-            sub[t] = a.fl[((1u << (a.L + l)) - 1) + (b << l) + p];
-        }
-    }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < c; i += BT) {
         const ulonglong2 e = ent[i];
@@ -765,7 +760,7 @@ cudaError_t part_prepare() {
 // When the partitioned front takes a batch of n keys, and with how many
 // buckets of which capacity.
 PartPlan part_plan(uint64_t n, uint32_t H) {
-    PartPlan p{0, 0, 0};
+    PartPlan p{};
     if (n < PART_MIN || n > PART_MAX || H < 9) return p;
     // Buckets of 32 keys as long as every one has an SM to itself (against
     // 128 keys: calls of 1,000 to 5,000 keys 66-70 us instead of 71-83),
@@ -789,6 +784,9 @@ PartPlan part_plan(uint64_t n, uint32_t H) {
     if (cap > 4096) return p;  // a batch that is large against the tree
     p.L = L;
     p.cap = (uint32_t)cap;
+    // a bucket of few keys stages its subtree only where that costs others
+    // nothing: the descents of 32 keys through 14 levels in L2 took 7 us
+    p.stage = L <= PART_WAVE || avg >= 64;
     p.ipt = (uint32_t)std::min<uint64_t>(PART_IPT, std::max<uint64_t>(1, n / (PT * PART_GRID)));
     return p;
 }

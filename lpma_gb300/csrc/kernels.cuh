@@ -53,6 +53,7 @@ struct PartPlan {
     uint32_t L;    // 2^L buckets; 0: the sorted front takes the batch
     uint32_t cap;  // entries of a bucket
     uint32_t ipt;  // keys a thread of the partition takes
+    bool stage;    // the buckets stage their subtrees
 };
 PartPlan part_plan(uint64_t n, uint32_t H);
 struct PartArgs {
@@ -64,8 +65,6 @@ struct PartArgs {
     const ulonglong2 *fl;
     ulonglong2 *ent;  // 2^L buckets of cap entries (key, payload)
     uint32_t *fill;   // entries of each bucket (zero before)
-    uint32_t *bitmap;
-    uint32_t bitmap_words;
     DevStatus *st;
 };
 struct BucketArgs {
@@ -79,6 +78,8 @@ struct BucketArgs {
     uint32_t *pcnt;     // per bucket: updates left (low half) and inserts among them
     uint32_t *bwin;     // per bucket: single-segment windows executed
     uint32_t *absbits;  // bit s + 1: segment s was executed
+    uint32_t *bitmap;   // the planner's, cleared here
+    uint32_t bitmap_words, stage;  // stage: the subtree's top levels go to shared memory
     DevStatus *st;
 };
 // the partition kernel's entry (graph replays replace its arguments)
