@@ -687,7 +687,9 @@ lpma_status_t enqueue_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, 
     launch_pack(ins, ins_vals, (uint32_t)n_ins, del, (uint32_t)n_del, h->V, thres, key_format, internal ? 1 : 0,
                 h->bk0, h->bp0, h->dst, h->c.bitmap, (uint32_t)bitmap_words(h->H), h->c.fl, h->c.cnt,
                 prefetch_segs(h, n), h->sup, sup_words_for(n), h->sort.bar, s);
-    if (thres_active) launch_live_counts(h->c.keys, h->H, thres, h->c.cnt_live, h->dst, s);
+    // from here on every kernel takes the threshold from the status block
+    thres = thres ? THRES_IN_STATUS : 0;
+    if (thres_active) launch_live_counts(h->c.keys, h->c.cnt, h->H, thres, h->c.cnt_live, h->dst, s);
     // sort (digit bytes decided on the device), resolve + locate, compact
     const SortTier tier = sort_tier_for_update((uint32_t)n, h->sort);
     const SortMask mask = update_sort_mask(&h->dst->key_and, tier, (uint32_t)n, h->sort);
@@ -739,6 +741,7 @@ lpma_status_t enqueue_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, 
     if (fork) CK(cudaEventRecord(h->join_ev, side));
     launch_exec_single(h->wsingle, (uint32_t)n, ge, h->c.cnt, h->c.fl, h->sent, h->V, h->u, thres, h->dst, s, true);
     if (fork) CK(cudaStreamWaitEvent(s, h->join_ev, 0));
+    if (pub && thres_active) launch_sum_cnt(h->c.cnt, nseg_of(h->H), h->dst, s, h->hst_dev);
     return LPMA_OK;
 }
 
@@ -748,11 +751,12 @@ lpma_status_t enqueue_part(LpmaHandle *h, cudaStream_t s, const PartArgs &pa, si
                            bool thres_active) {
     CK(cudaMemcpyAsync(h->dst, h->hinit, offsetof(DevStatus, sticky), cudaMemcpyHostToDevice, s));
     launch_part(pa, s);
-    if (thres_active) launch_live_counts(h->c.keys, h->H, pa.thres, h->c.cnt_live, h->dst, s);
+    const uint32_t thres = pa.thres ? THRES_IN_STATUS : 0;
+    if (thres_active) launch_live_counts(h->c.keys, h->c.cnt, h->H, thres, h->c.cnt_live, h->dst, s);
     Tables tb = make_tables(h, h->H, true);
     set_grain(tb, n);
     const Geo g{h->c.keys, h->c.vals, h->H};
-    const BucketArgs ba{g, h->c.fl, h->c.cnt, thres_active ? h->c.cnt_live : nullptr, h->sent, h->V, pa.thres,
+    const BucketArgs ba{g, h->c.fl, h->c.cnt, thres_active ? h->c.cnt_live : nullptr, h->sent, h->V,
                         tb.lower[0], pp.L, pp.cap, h->part_ent, pa.fill, pa.fill + (1u << PART_L_MAX),
                         pa.fill + (2u << PART_L_MAX), h->c.absbits, h->c.bitmap, (uint32_t)bitmap_words(h->H),
                         pp.stage, h->dst};
@@ -775,8 +779,9 @@ lpma_status_t enqueue_part(LpmaHandle *h, cudaStream_t s, const PartArgs &pa, si
                                 cs == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault));
     if (fork) CK(cudaEventRecord(h->join_ev, side));
     launch_exec_multi(h->wsmall4, (uint32_t)n, h->wsmall, (uint32_t)n, g, h->c.cnt, h->c.fl, h->sent, h->V, h->u,
-                      pa.thres, h->dst, s, true);
+                      thres, h->dst, s, true);
     if (fork) CK(cudaStreamWaitEvent(s, h->join_ev, 0));
+    if (pub && thres_active) launch_sum_cnt(h->c.cnt, nseg_of(h->H), h->dst, s, h->hst_dev);
     return LPMA_OK;
 }
 
@@ -831,6 +836,8 @@ lpma_status_t run_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, cons
     // the stored-key count reaches the planner through the status reset copy,
     // so that it is not a kernel argument of a cached graph
     h->hinit->total_items = h->total;
+    h->hinit->thres = thres;
+    h->hinit->seq++;
     const PartPlan pp = plan_part(h, n, internal);
     h->front_part = pp.L != 0;
     if (pp.L) CKS(ensure_part(h, pp, s));
@@ -844,7 +851,7 @@ lpma_status_t run_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, cons
     if (internal || prof_enabled() || !graphs_enabled()) {
         CKS(enqueue(s));
     } else {
-        const uint64_t key[12] = {n_ins, n_del, h->H, thres,
+        const uint64_t key[12] = {n_ins, n_del, h->H, thres != 0,
                                   (uint64_t)thres_active | ((uint64_t)(ins_vals != nullptr) << 1) |
                                       ((uint64_t)(h->sort.bar != nullptr) << 2) |
                                       ((uint64_t)sort_tier_for_update((uint32_t)n, h->sort) << 3) |
@@ -957,14 +964,18 @@ void mark_done(LpmaHandle *h, cudaStream_t s) {
 // queried now and then, it ends the wait with the error of a failed kernel,
 // or, should the word not be seen once the planner has finished, the status
 // is copied back instead.
-cudaError_t wait_published(LpmaHandle *h) {
+// recount: for the `counted` word instead, which the recount behind the
+// executors on stream s sets.
+cudaError_t wait_published(LpmaHandle *h, bool recount = false, cudaStream_t s = nullptr) {
+    uint32_t *flag = recount ? &h->hst->counted : &h->hst->published;
+    const uint32_t want = recount ? h->hinit->seq : 1u;
     for (uint32_t spin = 1;; spin++) {
-        if (__atomic_load_n(&h->hst->published, __ATOMIC_ACQUIRE)) return cudaSuccess;
+        if (__atomic_load_n(flag, __ATOMIC_ACQUIRE) == want) return cudaSuccess;
         if (spin % 64) continue;
-        const cudaError_t q = cudaEventQuery(h->front_ev);
+        const cudaError_t q = recount ? cudaStreamQuery(s) : cudaEventQuery(h->front_ev);
         if (q == cudaErrorNotReady) continue;
         if (q != cudaSuccess) return q;
-        if (__atomic_load_n(&h->hst->published, __ATOMIC_ACQUIRE)) return cudaSuccess;
+        if (__atomic_load_n(flag, __ATOMIC_ACQUIRE) == want) return cudaSuccess;
         const cudaError_t e = cudaMemcpyAsync(h->hst, h->dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, h->side_stream);
         return e ? e : cudaStreamSynchronize(h->side_stream);
     }
@@ -985,9 +996,11 @@ lpma_status_t wait_front(LpmaHandle *h, cudaStream_t) {
 // root / overflow / resize paths and the stats.  Shared by lpma_update and
 // the graphs of a batched update.  small_done: the first loop's single / 4 /
 // 32-segment executors already ran (in lpma_update's front, guarded, or in
-// the shared launches of a batched update).
+// the shared launches of a batched update).  front_counts: so is the recount
+// that a call with an expiry threshold ends with.
 lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t thres, bool thres_active,
-                            cudaStream_t s, LpmaStats &st, LpmaStats *out, bool small_done = false) {
+                            cudaStream_t s, LpmaStats &st, LpmaStats *out, bool small_done = false,
+                            bool front_counts = false) {
     // a sort that gave up a bounded wait turned the front into a no-op:
     // nothing changed, so the handle stays usable
     if (rs == LPMA_ERR_TIMEOUT && h->hst->sticky == 0) return rs;
@@ -1022,6 +1035,7 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
     st.n_noop = h->hst->n_noop;
     const int64_t live_after = live_before - n_gone + n_new;
 
+    const bool front_ovf = h->hst->ovf != 0, front_big = h->hst->n_big != 0;
     lpma_status_t r = LPMA_OK;
     if (n_new + n_gone > 0 && !h->hst->ovf) {
         const bool root = h->hst->root != 0;
@@ -1053,7 +1067,7 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
                 launch_relocate(h->u2, n2, g2, h->c.fl, s);
                 if (thres_active) {
                     CK(cudaMemsetAsync(&h->dst->live_total, 0, 8, s));
-                    launch_live_counts(h->c.keys, h->H, thres, h->c.cnt_live, h->dst, s);
+                    launch_live_counts(h->c.keys, h->c.cnt, h->H, thres, h->c.cnt_live, h->dst, s);
                 }
                 Tables tb2 = make_tables(h, h->H, false);
                 set_grain(tb2, n);
@@ -1070,7 +1084,7 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
                         launch_check_empty_level(h->c.cnt, h->H, h->dst, s);
                         r = sync_status(h, s);
                         if (r == LPMA_OK && h->hst->empty_found) {
-                            if (thres_active) launch_live_counts(h->c.keys, h->H, thres, h->c.cnt_live, h->dst, s);
+                            if (thres_active) launch_live_counts(h->c.keys, h->c.cnt, h->H, thres, h->c.cnt_live, h->dst, s);
                             r = rebuild(h, h->H, h->u2, 0, (uint64_t)live_after, thres, thres_active, s, &st);
                             st.rebuilt = 0;
                             st.fill_empty = 1;
@@ -1084,7 +1098,13 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
         }
     }
     if (r != LPMA_OK) return h->sticky = r;
-    if (thres_active) {
+    if (thres_active && front_counts && !front_ovf && !front_big) {
+        // recounted behind the front's executors, which did everything
+        CK(wait_published(h, true, s));
+        h->d2h += 16;
+        if (h->hst->sticky & (ERR_TIMEOUT | ERR_INTERNAL))
+            return h->sticky = (h->hst->sticky & ERR_TIMEOUT) ? LPMA_ERR_TIMEOUT : LPMA_ERR_INTERNAL;
+    } else if (thres_active) {
         // executed windows dropped expired keys: recount what is stored
         CK(cudaMemsetAsync(&h->dst->cnt_total, 0, 8, s));
         launch_sum_cnt(h->c.cnt, nseg_of(h->H), h->dst, s);
@@ -1140,7 +1160,7 @@ lpma_status_t do_update(LpmaHandle *h, const uint64_t *ins, const uint8_t *ins_v
         CKS(run_front(h, s, ins, ins_vals, n_ins, del, n_del, thres, thres_active, internal));
         rs = wait_front(h, s);
     }
-    return finish_update(h, rs, n, thres, thres_active, s, st, out, true);
+    return finish_update(h, rs, n, thres, thres_active, s, st, out, true, front_publishes(h));
 }
 
 }  // namespace
@@ -1434,6 +1454,7 @@ lpma_status_t lpma_create(const LpmaConfig *cfg, uint32_t num_vertices, lpma_str
         cudaGetLastError();
     }
     std::memset(h->hinit, 0, sizeof(DevStatus));
+    std::memset(h->hst, 0, sizeof(DevStatus));  // its block may have been another handle's
     h->hinit->min_t_ins = 0xFFFFFFFFu;
     h->hinit->key_and = ~0ull;
     h->hinit->err_info[0] = 0xFFFFFFFFu;

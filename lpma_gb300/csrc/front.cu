@@ -276,6 +276,7 @@ __global__ void __launch_bounds__(BT, BUCKET_CTAS) k_bucket(BucketArgs a) {
     griddep_wait();
     // a rejected batch, or one whose buckets overflowed, changes nothing
     if (a.st->error | a.st->part_ovf) return;
+    const uint32_t thres = TH ? a.st->thres : 0;
     const uint32_t c = min(a.fill[b], a.cap);
     for (uint32_t i = threadIdx.x; i < W / 32; i += BT) bits[i] = 0;
     if (threadIdx.x < 8) F.stat[threadIdx.x] = 0;
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(BT, BUCKET_CTAS) k_bucket(BucketArgs a) {
                     kd = KIND_INS;
                     atomicAdd(&sc[t], 1u);
                 }
-            } else if (found && (!TH || (key & TIME_MASK) >= (uint64_t)a.thres)) {
+            } else if (found && (!TH || (key & TIME_MASK) >= (uint64_t)thres)) {
                 a.g.vals[slot0 + rank] = VAL_TOMB;  // until a window executes
                 kd = KIND_DEL;
                 atomicAdd(&sc[t], 1u << 16);
@@ -558,7 +559,7 @@ __global__ void __launch_bounds__(BT, BUCKET_CTAS) k_bucket(BucketArgs a) {
 #pragma unroll
             for (int q = 0; q < 8; q++) {
                 const uint8_t v = (uint8_t)(v8 >> (8 * q));
-                if (k[q] != KEY_NONE && !(TH ? kept_slot(k[q], v, a.thres) : v != VAL_TOMB)) dm |= 1u << q;
+                if (k[q] != KEY_NONE && !(TH ? kept_slot(k[q], v, thres) : v != VAL_TOMB)) dm |= 1u << q;
             }
             dm <<= 8 * gl;
             dm |= __shfl_xor_sync(0xffffffffu, dm, 1, 4);

@@ -72,7 +72,7 @@ struct BucketArgs {
     ulonglong2 *fl;
     uint8_t *cnt, *cnt_live;  // cnt_live: with an active expiry threshold, else null
     uint32_t *sent;
-    uint32_t V, thres, lower0, L, cap;
+    uint32_t V, lower0, L, cap;
     ulonglong2 *ent;
     uint32_t *fill;
     uint32_t *pcnt;     // per bucket: updates left (low half) and inserts among them
@@ -90,8 +90,9 @@ void launch_part(const PartArgs &a, cudaStream_t s);
 void launch_buckets(const BucketArgs &a, const UpdList &u, cudaStream_t s);
 
 // per-segment live counts (key present and t >= thres) + their total
-void launch_live_counts(const uint64_t *keys, uint32_t H, uint32_t thres, uint8_t *cnt_live, DevStatus *st,
-                        cudaStream_t s);
+// (cnt: the segments' stored counts)
+void launch_live_counts(const uint64_t *keys, const uint8_t *cnt, uint32_t H, uint32_t thres, uint8_t *cnt_live,
+                        DevStatus *st, cudaStream_t s);
 
 // collapse duplicates, locate every key, membership test against its
 // segment, upsert/tombstone in place; per-256-block counts of kept entries
@@ -195,7 +196,7 @@ void launch_set_job(TileJob *jobs, const TileJob &j, cudaStream_t s);
 // new level: cnt re-index (old s -> 2s+1), empty leaves
 void launch_levelup_cnt(const uint8_t *cnt_old, uint8_t *cnt_new, uint32_t H_old, cudaStream_t s);
 void launch_check_empty_level(const uint8_t *cnt, uint32_t H, DevStatus *st, cudaStream_t s);
-void launch_sum_cnt(const uint8_t *cnt, uint64_t nseg, DevStatus *st, cudaStream_t s);
+void launch_sum_cnt(const uint8_t *cnt, uint64_t nseg, DevStatus *st, cudaStream_t s, DevStatus *pub = nullptr);
 
 // view
 // the CSR view (and / or the export) of the tree; tiles: one word per 128

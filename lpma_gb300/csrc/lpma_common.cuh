@@ -101,6 +101,9 @@ struct DevStatus {
     uint32_t abs_ins, abs_del;       // inserts and deletes of the abs_win windows
     uint32_t part_ovf;               // a bucket overflowed: nothing was done, the sorted front takes the batch
     uint32_t plan_done;              // planner CTAs finished (the front's status publish)
+    uint32_t thres;                  // the call's expiry threshold (set by the host)
+    uint32_t seq;                    // the call's number (set by the host)
+    uint32_t sum_done;               // recount CTAs finished
     // Not reset per call (the reset copies the fields above only): the
     // executors set ERR_INTERNAL here after the call may have returned.
     uint32_t sticky;
@@ -108,7 +111,12 @@ struct DevStatus {
     // Meaningful in the host mirror only: set to 1 by the planner's last CTA
     // after it wrote the words above into the mirror (k_plan_max, publish).
     uint32_t published;
+    uint32_t counted;  // set to seq by the recount behind the executors (k_sum_cnt, pub)
 };
+// As a kernel's threshold argument: the one in the status block.  A captured
+// front then serves calls of every threshold; a stream of ticks passes
+// another one each call.
+constexpr uint32_t THRES_IN_STATUS = ~0u;
 
 // A rebalance window chosen by the planner (maximal executed window); 8-byte
 // aligned so that a record loads as three 64-bit words.

@@ -224,18 +224,44 @@ __global__ void __launch_bounds__(TPB) k_pack(const uint64_t *__restrict__ ins, 
 }
 
 // ------------------------------------------------------------------ live counts
-__global__ void __launch_bounds__(TPB) k_live_counts(const uint64_t *__restrict__ keys, uint32_t H, uint32_t thres,
-                                                     uint8_t *cnt_live, DevStatus *st) {
-    const uint64_t nseg = nseg_of(H);
-    const int lane = threadIdx.x & 31;
+// Bound by HBM: the occupied part of every segment once.  8 lanes a segment,
+// 4 slots each, so that a warp has 16 segments in flight: 262,143 segments
+// with 21 keys each took 27 us a warp and a whole row each, 14 so.
+__global__ void __launch_bounds__(TPB) k_live_counts(const uint64_t *__restrict__ keys, const uint8_t *__restrict__ cnt,
+                                                     uint32_t H, uint32_t thres, uint8_t *cnt_live, DevStatus *st) {
+    if (thres == THRES_IN_STATUS) thres = st->thres;
+    const uint32_t nseg = (uint32_t)nseg_of(H);
+    const int lane = threadIdx.x & 31, gl = lane & 7;
+    constexpr uint32_t U = 4;
+    const uint32_t step = gridDim.x * (TPB / 32) * 4 * U;
     uint32_t acc = 0;
-    for (uint64_t s = (blockIdx.x * (uint64_t)TPB + threadIdx.x) >> 5; s < nseg; s += (gridDim.x * (uint64_t)TPB) >> 5) {
-        uint64_t j = heap_of_linear(s, H);
-        uint64_t k = keys[32 * j + lane];
-        uint32_t c = __popc(__ballot_sync(0xffffffffu, k != KEY_NONE && (k & TIME_MASK) >= (uint64_t)thres));
-        if (lane == 0) cnt_live[s] = (uint8_t)c;
-        acc += c;
+    for (uint32_t s0 = (blockIdx.x * (TPB / 32) + (threadIdx.x >> 5)) * 4 * U + (lane >> 3);; s0 += step) {
+        if (s0 - (lane >> 3) >= nseg) break;  // uniform over the warp
+        uint32_t c[U];
+        ulonglong2 a[U], b[U];
+#pragma unroll
+        for (uint32_t q = 0; q < U; q++) c[q] = s0 + 4 * q < nseg ? cnt[s0 + 4 * q] : 0u;
+#pragma unroll
+        for (uint32_t q = 0; q < U; q++) {
+            a[q] = b[q] = make_ulonglong2(KEY_NONE, KEY_NONE);
+            if (4u * gl < c[q]) {
+                const uint64_t j = heap_of_linear32(s0 + 4 * q, H);
+                const ulonglong2 *kp = reinterpret_cast<const ulonglong2 *>(keys + 32 * j + 4 * gl);
+                a[q] = kp[0], b[q] = kp[1];
+            }
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < U; q++) {
+            auto live = [&](uint64_t k) { return (k != KEY_NONE && (k & TIME_MASK) >= (uint64_t)thres) ? 1u : 0u; };
+            uint32_t x = live(a[q].x) + live(a[q].y) + live(b[q].x) + live(b[q].y);
+            acc += x;
+            x += __shfl_xor_sync(0xffffffffu, x, 1);
+            x += __shfl_xor_sync(0xffffffffu, x, 2);
+            x += __shfl_xor_sync(0xffffffffu, x, 4);
+            if (gl == 0 && s0 + 4 * q < nseg) cnt_live[s0 + 4 * q] = (uint8_t)x;
+        }
     }
+    acc = __reduce_add_sync(0xffffffffu, acc);
     if (lane == 0 && acc) atomicAdd(&st->live_total, (unsigned long long)acc);
 }
 
@@ -338,6 +364,7 @@ __global__ void __launch_bounds__(TPB) k_resolve_locate(const uint64_t *__restri
                                                         uint8_t *kind, uint32_t *seg, uint32_t *blk_nn,
                                                         uint32_t *blk_ins, uint32_t *sup, DevStatus *st) {
     griddep_wait();
+    if (thres == THRES_IN_STATUS) thres = st->thres;
     k_resolve_locate_body(k0, p0, k1, p1, n, mask, g, fl, thres, kind, seg, blk_nn, blk_ins, sup, st, blockIdx.x,
                           gridDim.x);
 }
@@ -1444,6 +1471,7 @@ __global__ void __launch_bounds__(EM_TPB, 4) k_exec_multi(const Window *__restri
     __shared__ __align__(16) unsigned char smem[EM_SMEM];
     griddep_wait();
     if (guarded && plan_void(st)) return;
+    if (thres == THRES_IN_STATUS) thres = st->thres;
     const uint32_t nb32 = gridDim.x - nb4;
     if (blockIdx.x < nb32)
         exec_multi32<TH>(smem, w32, n32, cap32, g, cnt, fl, sent, V, u, thres, st, blockIdx.x, nb32);
@@ -1625,6 +1653,7 @@ __global__ void __launch_bounds__(ES_TPB, 4) k_exec_single(const Window *__restr
                                                         int guarded) {
     griddep_wait();
     if (guarded && plan_void(st)) return;
+    if (thres == THRES_IN_STATUS) thres = st->thres;
     k_exec_single_body<TH>(wins, n_win, n_cap, g, cnt, fl, sent, V, u, thres, st, blockIdx.x, gridDim.x);
 }
 
@@ -2387,11 +2416,36 @@ __global__ void __launch_bounds__(TPB) k_check_empty_level(const uint8_t *__rest
         if (cnt[4 * t + 1] == 0) st->empty_found = 1;
 }
 
-__global__ void __launch_bounds__(TPB) k_sum_cnt(const uint8_t *__restrict__ cnt, uint64_t nseg, DevStatus *st) {
+// Stored keys after a call with an expiry threshold.  pub: the last CTA puts
+// the sum and the sticky words into the host's mirror and then sets its
+// `counted` word to the call's number (an earlier call may have returned,
+// rejected, before its recount).
+__global__ void __launch_bounds__(TPB) k_sum_cnt(const uint8_t *__restrict__ cnt, uint64_t nseg, DevStatus *st,
+                                                 DevStatus *pub) {
     uint32_t acc = 0;
-    for (uint64_t s = blockIdx.x * (uint64_t)TPB + threadIdx.x; s < nseg; s += gridDim.x * (uint64_t)TPB) acc += cnt[s];
+    const uint64_t whole = nseg / 16;
+    for (uint64_t i = blockIdx.x * (uint64_t)TPB + threadIdx.x; i < whole; i += gridDim.x * (uint64_t)TPB) {
+        const uint4 v = reinterpret_cast<const uint4 *>(cnt)[i];
+        acc = __dp4a(v.x, 0x01010101u, acc);
+        acc = __dp4a(v.y, 0x01010101u, acc);
+        acc = __dp4a(v.z, 0x01010101u, acc);
+        acc = __dp4a(v.w, 0x01010101u, acc);
+    }
+    if (blockIdx.x == 0 && threadIdx.x < nseg % 16) acc += cnt[16 * whole + threadIdx.x];
     acc = warp_sum(acc);
     if ((threadIdx.x & 31) == 0 && acc) atomicAdd(&st->cnt_total, (unsigned long long)acc);
+    if (pub == nullptr) return;  // uniform over the grid
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x || atomicAdd(&st->sum_done, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    const volatile DevStatus *src = st;
+    volatile DevStatus *dst = pub;
+    dst->cnt_total = src->cnt_total;
+    dst->sticky = src->sticky;
+    dst->sticky_site = src->sticky_site;
+    __threadfence_system();
+    dst->counted = src->seq;
 }
 
 inline uint32_t grid_for(uint64_t n, uint32_t per_block, uint32_t cap = 152 * 16) {
@@ -2418,10 +2472,10 @@ void launch_pack(const uint64_t *ins, const uint8_t *ins_vals, uint32_t n_ins, c
     note_launch();
 }
 
-void launch_live_counts(const uint64_t *keys, uint32_t H, uint32_t thres, uint8_t *cnt_live, DevStatus *st,
+void launch_live_counts(const uint64_t *keys, const uint8_t *cnt, uint32_t H, uint32_t thres, uint8_t *cnt_live, DevStatus *st,
                         cudaStream_t s) {
     ProfScope ps_("live_counts", s);
-    k_live_counts<<<grid_for(nseg_of(H), TPB / 32), TPB, 0, s>>>(keys, H, thres, cnt_live, st);
+    k_live_counts<<<grid_for(nseg_of(H), TPB / 2, 152 * 8), TPB, 0, s>>>(keys, cnt, H, thres, cnt_live, st);
     note_launch();
 }
 
@@ -2666,9 +2720,9 @@ void launch_check_empty_level(const uint8_t *cnt, uint32_t H, DevStatus *st, cud
     note_launch();
 }
 
-void launch_sum_cnt(const uint8_t *cnt, uint64_t nseg, DevStatus *st, cudaStream_t s) {
+void launch_sum_cnt(const uint8_t *cnt, uint64_t nseg, DevStatus *st, cudaStream_t s, DevStatus *pub) {
     ProfScope ps_("sum_cnt", s);
-    k_sum_cnt<<<grid_for(nseg, TPB), TPB, 0, s>>>(cnt, nseg, st);
+    k_sum_cnt<<<grid_for(nseg / 16, TPB, 152 * 2), TPB, 0, s>>>(cnt, nseg, st, pub);
     note_launch();
 }
 

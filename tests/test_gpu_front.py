@@ -174,3 +174,25 @@ def test_expiry_thresholds(engine, oracle, batch):
             dels = rng.choice(live, min(b // 5, live.size), replace=False)  # some have expired
         t.update(ins=keys, dels=dels, thres=max(0, tick - 5), where="tick %d" % tick)
     t.close()
+
+
+@pytest.mark.parametrize("batch", [100, 2000])
+def test_expiry_of_equal_batches(engine, oracle, batch):
+    """A threshold that moves with every call while the batch's shape stays
+    (one captured front serves them all), with a rejected call in between."""
+    from lpma_gb300 import LpmaError
+    V = 1 << 11
+    t = Three(engine, oracle, V)
+    rng = np.random.default_rng(batch)
+    edges = oracle.shuffle(oracle.rmat_edges(batch, 11, 24), 5)
+    edges = np.unique((edges >> DST) << DST)
+    edges = rng.permutation(edges)[: 14 * batch].reshape(14, batch)
+    for tick in range(1, 29):
+        ins = edges[tick % 14] | np.uint64(tick)
+        s = t.update(ins=ins, thres=max(0, tick - 6), where="tick %d" % tick)
+        assert s["n_ins_applied"] == batch
+        if tick == 15:
+            bad = np.append(ins[1:], _key([V], [0]))
+            with pytest.raises(LpmaError):
+                t.g.update(ins=_dev(bad), thres=tick - 6)
+    t.close()
