@@ -307,7 +307,7 @@ LPMA_API lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *grap
  * sorted by all-pairs rank over many CTAs, then placed by binary searches
  * across the tiles (<= 16384), 3 register-sorted tiles plus
  * merge-path rounds (<= 2^24), 4 one cooperative launch for all digit
- * passes (handles without LPMA_FLAG_CONCURRENT), 5 three launches per digit
+ * passes (handles without LPMA_FLAG_CONCURRENT), 5 one launch per digit
  * pass.  All give the same order.  lpma_autotune times every usable tier on
  * seeded batches of 2^b keys for b = 11 .. ceil(log2 max_keys), for both
  * sort modes (concurrent 0: cooperative launches allowed, 1: not), keeps

@@ -1,13 +1,11 @@
 // Radix sort and scan primitives (hand-written, sm_103a).
 //
-// Sort: LSD radix sort on 8-bit digits, reduce-then-scan per digit pass:
-// k_upsweep counts the digits of every 2048-key tile, k_dscan turns the
-// (digit, tile) counts into exclusive global offsets (digit-major, one warp
-// per digit, digit bases from a histogram of all eight digits taken once
-// per sort), k_downsweep ranks each tile's keys stably with
-// __match_any_sync and scatters them.  No CTA waits on another.  Bytes that
-// are equal across all keys are skipped.  Batches of at most one tile are
-// sorted by one CTA in shared memory in a single launch.
+// Sort: LSD radix sort on 8-bit digits, one launch per digit pass: k_hist
+// counts all digits once, k_onesweep ranks a tile's keys stably with ballots,
+// finds the tile's places from the counts that the tiles before it have
+// published and scatters the keys.  Bytes that are equal across all keys are
+// skipped.  Batches of at most 2,048 keys are sorted by one CTA in shared
+// memory in a single launch.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -236,14 +234,23 @@ __device__ inline void warp_rank(const uint64_t (&k)[IPT], uint32_t valid_mask, 
 }
 
 // ---------------------------------------------------------------- histogram
-__global__ void __launch_bounds__(256) k_hist(const uint64_t *__restrict__ keys, uint32_t n, uint32_t *hist) {
+__global__ void __launch_bounds__(256) k_hist(const uint64_t *__restrict__ keys, uint32_t n, uint32_t *hist,
+                                              SortMask mask) {
     __shared__ uint32_t h[8][256];
+    const uint32_t act = active_bytes(mask);
     for (int i = threadIdx.x; i < 8 * 256; i += 256) (&h[0][0])[i] = 0;
     __syncthreads();
-    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
-        const uint64_t k = keys[i];
+    for (uint64_t i0 = blockIdx.x * 1024ull + threadIdx.x; i0 < n; i0 += gridDim.x * 1024ull) {
+        uint64_t k[4];
 #pragma unroll
-        for (int b = 0; b < 8; b++) atomicAdd(&h[b][(k >> (8 * b)) & 0xFF], 1u);
+        for (int q = 0; q < 4; q++) k[q] = i0 + 256 * q < n ? keys[i0 + 256 * q] : 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (i0 + 256 * q >= n) break;
+#pragma unroll
+            for (int b = 0; b < 8; b++)
+                if ((act >> b) & 1u) atomicAdd(&h[b][(k[q] >> (8 * b)) & 0xFF], 1u);
+        }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < 8 * 256; i += 256) {
@@ -253,67 +260,39 @@ __global__ void __launch_bounds__(256) k_hist(const uint64_t *__restrict__ keys,
 }
 
 // ---------------------------------------------------------------- one pass
-__global__ void __launch_bounds__(SORT_TPB) k_upsweep(const uint64_t *__restrict__ k0, const uint64_t *__restrict__ k1,
-                                                      uint32_t n, int byte, SortMask mask, uint32_t *counts,
-                                                      uint32_t T) {
-    const uint32_t act = active_bytes(mask);
-    if (!((act >> byte) & 1u)) return;
-    const uint64_t *keys = (__popc(act & ((1u << byte) - 1)) & 1) ? k1 : k0;
-    const int sh = 8 * byte;
-    __shared__ uint32_t h[256];
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    const uint64_t base = (uint64_t)blockIdx.x * SORT_TILE;
-#pragma unroll
-    for (int i = 0; i < SORT_IPT; i++) {
-        const uint64_t p = base + (uint64_t)i * SORT_TPB + threadIdx.x;
-        if (p < n) atomicAdd(&h[(keys[p] >> sh) & 0xFF], 1u);
-    }
-    __syncthreads();
-    counts[(size_t)threadIdx.x * T + blockIdx.x] = h[threadIdx.x];
-}
-
-// one warp per digit: offs[d][t] = base(d) + sum of counts[d][t' < t]
-__global__ void __launch_bounds__(256) k_dscan(const uint32_t *__restrict__ counts, uint32_t T,
-                                               const uint32_t *__restrict__ hist, uint32_t *offs, int byte,
-                                               SortMask mask) {
-    if (!((active_bytes(mask) >> byte) & 1u)) return;
-    __shared__ uint32_t gd[256];
-    __shared__ uint32_t wsum[8];
-    gd[threadIdx.x] = block_excl_scan_256(hist[threadIdx.x], wsum, nullptr);
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const uint32_t d = blockIdx.x * 8 + (threadIdx.x >> 5);
-    uint32_t run = gd[d];
-    const uint32_t *c = counts + (size_t)d * T;
-    uint32_t *o = offs + (size_t)d * T;
-    for (uint32_t t0 = 0; t0 < T; t0 += 32) {
-        const uint32_t t = t0 + lane;
-        const uint32_t x = t < T ? c[t] : 0;
-        uint32_t v = x;
-#pragma unroll
-        for (int k = 1; k < 32; k <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, v, k);
-            if (lane >= k) v += y;
-        }
-        if (t < T) o[t] = run + v - x;
-        run += __shfl_sync(0xffffffffu, v, 31);
-    }
-}
+// A digit pass in one launch.  Tiles are handed out in order; a tile counts
+// its digits, publishes the counts, adds up those of the tiles before it (a
+// thread a digit, back to the nearest tile that has published its prefix)
+// while others do the same, publishes its own prefix and writes its keys.  A
+// tile waits only for lower ones, which are running and publish before they
+// wait; the wait is bounded all the same: after ONE_SPIN_LIMIT polls the sort
+// is marked as given up and the pass goes on, its writes within n.
+//
+// Bound by the ranking and the scatter, with HBM at half its rate.  One pass
+// over 16.8M keys: 154 us (160 with two CTAs an SM instead of three, 193 with
+// 6,144 keys a tile); counting, scanning the counts and ranking took three
+// launches, 50 + 39 + 113 us.
+constexpr int ONE_TPB = 512, ONE_IPT = 8, ONE_TILE = ONE_TPB * ONE_IPT, ONE_BACK = 4;
+constexpr uint32_t ONE_SPIN_LIMIT = 1u << 22;
+constexpr uint32_t ONE_SUM = 1u << 30, ONE_PREFIX = 2u << 30, ONE_VALUE = ONE_SUM - 1;  // n < 2^30
 
 template <typename V>
 struct PassSmem {
-    uint64_t k[SORT_TILE];
-    V v[SORT_TILE];
-    uint32_t whist[8][256];
-    uint32_t gbase[256];
+    uint64_t k[ONE_TILE];
+    V v[ONE_TILE];
+    uint32_t whist[ONE_TPB / 32][256];
+    uint32_t gbase[256];  // place of the digit's first key of the tile, less ldig
     uint32_t ldig[256];
     uint32_t wsum[8];
+    uint32_t tile;
 };
 
+// state: a word per digit of every tile, of this pass; cleared: the other
+// pass's, cleared here for the next one
 template <typename V>
-__global__ void __launch_bounds__(SORT_TPB) k_downsweep(uint64_t *k0, V *v0, uint64_t *k1, V *v1, uint32_t n, int byte,
-                                                        SortMask mask, const uint32_t *__restrict__ offs, uint32_t T) {
+__global__ void __launch_bounds__(ONE_TPB, 3) k_onesweep(uint64_t *k0, V *v0, uint64_t *k1, V *v1, uint32_t n, int byte,
+                                                      SortMask mask, const uint32_t *__restrict__ hist, uint32_t *state0,
+                                                      uint32_t *state1, uint32_t *next, uint32_t *err) {
     const uint32_t act = active_bytes(mask);
     if (!((act >> byte) & 1u)) return;
     const bool odd = __popc(act & ((1u << byte) - 1)) & 1;
@@ -321,21 +300,38 @@ __global__ void __launch_bounds__(SORT_TPB) k_downsweep(uint64_t *k0, V *v0, uin
     const V *__restrict__ vi = odd ? v1 : v0;
     uint64_t *__restrict__ ko = odd ? k0 : k1;
     V *__restrict__ vo = odd ? v0 : v1;
+    volatile uint32_t *state = odd ? state1 : state0;
+    uint32_t *other = odd ? state0 : state1;
     const int sh = 8 * byte;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PassSmem<V> &S = *reinterpret_cast<PassSmem<V> *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const uint32_t tile = blockIdx.x;
-    for (int i = tid; i < 8 * 256; i += SORT_TPB) (&S.whist[0][0])[i] = 0;
-    S.gbase[tid] = offs[(size_t)tid * T + tile];
-    __syncthreads();
-    const uint64_t base = (uint64_t)tile * SORT_TILE;
-    uint64_t k[SORT_IPT];
-    V v[SORT_IPT];
+    if (tid == 0) S.tile = atomicAdd(&next[byte], 1u);
+    for (int i = tid; i < (ONE_TPB / 32) * 256; i += ONE_TPB) (&S.whist[0][0])[i] = 0;
+    // exclusive sums over the digits (thread tid == digit, the upper half idle)
+    auto digit_scan = [&](uint32_t x) {
+        uint32_t y = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t z = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= o) y += z;
+        }
+        if (lane == 31 && w < 8) S.wsum[w] = y;
+        __syncthreads();
+        y -= x;
+        for (int q = 0; q < min(w, 8); q++) y += S.wsum[q];
+        __syncthreads();
+        return y;
+    };
+    const uint32_t dbase = digit_scan(tid < 256 ? hist[tid] : 0u);  // keys of smaller digits
+    const uint32_t tile = S.tile;
+    const uint64_t base = (uint64_t)tile * ONE_TILE;
+    uint64_t k[ONE_IPT];
+    V v[ONE_IPT];
     uint32_t vmask = 0;
 #pragma unroll
-    for (int i = 0; i < SORT_IPT; i++) {
-        const uint64_t p = base + (uint64_t)w * 32 * SORT_IPT + i * 32 + lane;
+    for (int i = 0; i < ONE_IPT; i++) {
+        const uint64_t p = base + (uint64_t)w * 32 * ONE_IPT + i * 32 + lane;
         if (p < n) {
             k[i] = ki[p];
             v[i] = vi[p];
@@ -345,21 +341,28 @@ __global__ void __launch_bounds__(SORT_TPB) k_downsweep(uint64_t *k0, V *v0, uin
             v[i] = V(0);
         }
     }
-    uint32_t rank[SORT_IPT];
-    warp_rank<SORT_IPT>(k, vmask, sh, S.whist[w], rank);
+    uint32_t rank[ONE_IPT];
+    warp_rank<ONE_IPT>(k, vmask, sh, S.whist[w], rank);
     __syncthreads();
     // per digit (thread tid == digit): warp-exclusive offsets and tile count
     uint32_t tcount = 0;
+    if (tid < 256) {
 #pragma unroll
-    for (int ww = 0; ww < 8; ww++) {
-        const uint32_t c = S.whist[ww][tid];
-        S.whist[ww][tid] = tcount;
-        tcount += c;
+        for (int ww = 0; ww < ONE_TPB / 32; ww++) {
+            const uint32_t c = S.whist[ww][tid];
+            S.whist[ww][tid] = tcount;
+            tcount += c;
+        }
+        state[(size_t)tile * 256 + tid] = tcount | (tile ? ONE_SUM : ONE_PREFIX);
+        other[(size_t)tile * 256 + tid] = 0;
     }
-    S.ldig[tid] = block_excl_scan_256(tcount, S.wsum, nullptr);
+    {
+        const uint32_t x = digit_scan(tcount);
+        if (tid < 256) S.ldig[tid] = x;
+    }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < SORT_IPT; i++) {
+    for (int i = 0; i < ONE_IPT; i++) {
         if ((vmask >> i) & 1u) {
             const uint32_t d = (uint32_t)((k[i] >> sh) & 0xFF);
             const uint32_t pos = S.ldig[d] + S.whist[w][d] + rank[i];
@@ -367,14 +370,43 @@ __global__ void __launch_bounds__(SORT_TPB) k_downsweep(uint64_t *k0, V *v0, uin
             S.v[pos] = v[i];
         }
     }
+    if (tid < 256) {
+        uint32_t before = 0, polls = 0;
+        int64_t t = (int64_t)tile - 1;
+        while (t >= 0) {
+            uint32_t x[ONE_BACK];  // some tiles back at once
+#pragma unroll
+            for (int q = 0; q < ONE_BACK; q++) x[q] = t >= q ? (uint32_t)state[(size_t)(t - q) * 256 + tid] : +ONE_PREFIX;
+            bool done = false, stuck = false;
+#pragma unroll
+            for (int q = 0; q < ONE_BACK; q++) {
+                if (done || stuck) continue;
+                if (x[q] == 0) {
+                    stuck = true;
+                } else {
+                    before += x[q] & ONE_VALUE;
+                    done = x[q] >= ONE_PREFIX;
+                    t--;
+                }
+            }
+            if (done) break;
+            if (stuck && ++polls > ONE_SPIN_LIMIT) {
+                if (err) atomicOr(err, ERR_TIMEOUT);
+                break;
+            }
+        }
+        if (tile) state[(size_t)tile * 256 + tid] = ((before + tcount) & ONE_VALUE) | ONE_PREFIX;
+        S.gbase[tid] = dbase + before - S.ldig[tid];
+    }
     __syncthreads();
-    const uint32_t nvalid = (uint32_t)umin64(SORT_TILE, n - base);
-    for (uint32_t p = tid; p < nvalid; p += SORT_TPB) {
+    const uint32_t nvalid = (uint32_t)umin64(ONE_TILE, n - base);
+    for (uint32_t p = tid; p < nvalid; p += ONE_TPB) {
         const uint64_t kk = S.k[p];
-        const uint32_t d = (uint32_t)((kk >> sh) & 0xFF);
-        const uint32_t g = S.gbase[d] + (p - S.ldig[d]);
-        ko[g] = kk;
-        vo[g] = S.v[p];
+        const uint32_t g = S.gbase[(uint32_t)((kk >> sh) & 0xFF)] + p;
+        if (g < n) {
+            ko[g] = kk;
+            vo[g] = S.v[p];
+        }
     }
 }
 
@@ -385,9 +417,7 @@ __global__ void __launch_bounds__(SORT_TPB) k_downsweep(uint64_t *k0, V *v0, uin
 // reordered in shared memory while the CTA waits); CTAs scan the count
 // columns (one digit each); grid barrier; every CTA adds its column offsets
 // to the global digit bases and writes its reordered tile out; grid
-// barrier before the next pass reads.  The
-// three grid barriers replace the reduce-then-scan sort's three launches
-// per digit and its separate histogram pass.  Every barrier wait is bounded:
+// barrier before the next pass reads.  Every barrier wait is bounded:
 // after BAR_SPIN_LIMIT polls the CTA records ERR_TIMEOUT and goes on, so
 // the kernel always ends.
 
@@ -1250,8 +1280,8 @@ static SortTier tier_default(uint32_t n, const SortScratch &s) {
     if (tier_ok<V>(TIER_COOP, n, s)) return TIER_COOP;
     if (n <= (uint32_t)SORT_TILE) return TIER_SMALL;
     // without a cooperative launch (concurrent handles) the merge rounds beat
-    // three launches per digit pass up to 2^19 keys (measured: 113 against
-    // 148 us at 2^19, 226 against 187 at 2^20)
+    // a launch per digit pass up to 2^19 keys (97 us against 110 at 2^19, 209
+    // against 137 at 2^20)
     if (n <= (1u << 19) && tier_ok<V>(TIER_TILE_MERGE, n, s)) return TIER_TILE_MERGE;
     return TIER_MULTIPASS;
 }
@@ -1346,32 +1376,26 @@ static cudaError_t sort_impl(uint64_t *k0, V *v0, uint64_t *k1, V *v1, uint32_t 
         note_launch();
         return cudaGetLastError();
     }
-    const uint32_t tiles = (n + SORT_TILE - 1) / SORT_TILE;
-    if (s.status_words < 2 * (size_t)tiles * 256) return cudaErrorInvalidValue;
-    uint32_t *counts = s.status, *offs = s.status + (size_t)tiles * 256;
+    const uint32_t tiles = (n + ONE_TILE - 1) / ONE_TILE;
+    const size_t words = (size_t)tiles * 256;
+    if (s.status_words < 2 * words) return cudaErrorInvalidValue;
+    uint32_t *next = s.counters + 8;  // tiles handed out, per pass
     if ((e = cudaMemsetAsync(s.hist, 0, 8 * 256 * sizeof(uint32_t), st))) return e;
-    const uint32_t hb = tiles < 1024 ? tiles : 1024;
+    if ((e = cudaMemsetAsync(next, 0, 8 * sizeof(uint32_t), st))) return e;
+    if ((e = cudaMemsetAsync(s.status, 0, words * sizeof(uint32_t), st))) return e;  // a pass clears the next one's
+    const uint32_t hb = std::min<uint32_t>((n + 2047) / 2048, 152 * 6);
     {
         ProfScope ps("sort_hist", st);
-        k_hist<<<hb, 256, 0, st>>>(k0, n, s.hist);
+        k_hist<<<hb, 256, 0, st>>>(k0, n, s.hist, mask);
     }
     note_launch();
     const size_t sm = sizeof(PassSmem<V>);
     for (int b = 0; b < 8; b++) {
         if (!((mask.host_mask >> b) & 1u)) continue;
-        {
-            ProfScope ps("sort_upsweep", st);
-            k_upsweep<<<tiles, SORT_TPB, 0, st>>>(k0, k1, n, b, mask, counts, tiles);
-        }
-        {
-            ProfScope ps("sort_dscan", st);
-            k_dscan<<<32, 256, 0, st>>>(counts, tiles, s.hist + 256 * b, offs, b, mask);
-        }
-        {
-            ProfScope ps("sort_downsweep", st);
-            k_downsweep<V><<<tiles, SORT_TPB, sm, st>>>(k0, v0, k1, v1, n, b, mask, offs, tiles);
-        }
-        note_launch(3);
+        ProfScope ps("sort_pass", st);
+        k_onesweep<V><<<tiles, ONE_TPB, sm, st>>>(k0, v0, k1, v1, n, b, mask, s.hist + 256 * b, s.status,
+                                                  s.status + words, next, s.err);
+        note_launch();
     }
     return cudaGetLastError();
 }
@@ -1413,10 +1437,10 @@ static cudaError_t sort_setup_device(int dev, CoopCtas &out) {
     if ((e = cudaFuncSetAttribute(k_small_sort<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sizeof(SmallSmem<uint64_t>))))
         return e;
-    if ((e = cudaFuncSetAttribute(k_downsweep<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if ((e = cudaFuncSetAttribute(k_onesweep<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sizeof(PassSmem<uint16_t>))))
         return e;
-    if ((e = cudaFuncSetAttribute(k_downsweep<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if ((e = cudaFuncSetAttribute(k_onesweep<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sizeof(PassSmem<uint64_t>))))
         return e;
     if ((e = cudaFuncSetAttribute(k_rank_merge, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -51,7 +51,7 @@ enum SortTier : uint32_t {
     TIER_BLOCK = 2,       // ranks: tiles of 2048 by all-pairs rank, then merged by binary searches, <= 16384 keys, in place
     TIER_TILE_MERGE = 3,  // register-sorted tiles + merge-path rounds, <= 2^24 keys, in place
     TIER_COOP = 4,        // one cooperative launch, all digit passes, ping-pong
-    TIER_MULTIPASS = 5,   // three launches per digit pass, ping-pong
+    TIER_MULTIPASS = 5,   // one launch per digit pass, ping-pong
     TIER_COUNT = 6
 };
 inline __host__ __device__ bool sort_tier_in_place(SortTier t) {
