@@ -573,6 +573,10 @@ __device__ __forceinline__ void k_compact_body(const uint64_t *__restrict__ k0, 
     }
 }
 
+// Four chunks a CTA (the counts of the chunks before are added up once for
+// them), one row of 32 entries a ballot.  16.8M keys: 244 us with one chunk a
+// CTA, 121 so.
+constexpr uint32_t CP_CHUNKS = 4;
 __global__ void __launch_bounds__(TPB) k_compact(const uint64_t *__restrict__ k0, const uint16_t *__restrict__ p0,
                                                  const uint64_t *__restrict__ k1, const uint16_t *__restrict__ p1,
                                                  SortMask mask, const uint8_t *__restrict__ kind,
@@ -580,7 +584,58 @@ __global__ void __launch_bounds__(TPB) k_compact(const uint64_t *__restrict__ k0
                                                  const uint32_t *blk_nn, const uint32_t *blk_ins,
                                                  const uint32_t *sup, UpdList u, DevStatus *st) {
     griddep_wait();
-    k_compact_body(k0, p0, k1, p1, mask, kind, seg, n, blk_nn, blk_ins, sup, u, st, blockIdx.x, gridDim.x);
+    const bool odd = sort_result_odd(mask, n);
+    const uint64_t *__restrict__ skey = odd ? k1 : k0;
+    const uint16_t *__restrict__ spay = odd ? p1 : p0;
+    __shared__ uint64_t wsum64[TPB / 32], own64[TPB / 32];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, lt = lanemask_lt();
+    const uint32_t c0 = blockIdx.x * CP_CHUNKS, grp = c0 / SUP_CHUNKS;
+    uint64_t acc = 0;  // kept entries before (low half), inserts among them (high half)
+    for (uint32_t t = threadIdx.x; t < grp; t += TPB) acc += (uint64_t)sup[2 * t] | ((uint64_t)sup[2 * t + 1] << 32);
+    for (uint32_t t = grp * SUP_CHUNKS + threadIdx.x; t < c0; t += TPB)
+        acc += (uint64_t)blk_nn[t] | ((uint64_t)blk_ins[t] << 32);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    const uint64_t i0 = (uint64_t)c0 * TPB + w * 32 * CP_CHUNKS + lane;
+    uint32_t kd[CP_CHUNKS], nn[CP_CHUNKS], ni[CP_CHUNKS], cn = 0, ci = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < CP_CHUNKS; q++) kd[q] = i0 + 32 * q < n ? kind[i0 + 32 * q] : KIND_NOP;
+#pragma unroll
+    for (uint32_t q = 0; q < CP_CHUNKS; q++) {
+        const uint32_t b = __ballot_sync(0xffffffffu, kd[q] != KIND_NOP);
+        const uint32_t bi = __ballot_sync(0xffffffffu, kd[q] == KIND_INS);
+        nn[q] = cn + __popc(b & lt), ni[q] = ci + __popc(bi & lt);
+        cn += __popc(b), ci += __popc(bi);
+    }
+    if (lane == 0) wsum64[w] = acc, own64[w] = (uint64_t)cn | ((uint64_t)ci << 32);
+    __syncthreads();
+    acc = 0;
+    uint64_t all = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < TPB / 32; q++) {
+        acc += wsum64[q] + (q < w ? own64[q] : 0ull);
+        all += wsum64[q] + own64[q];
+    }
+    const uint32_t bn = (uint32_t)acc, bi = (uint32_t)(acc >> 32);
+#pragma unroll
+    for (uint32_t q = 0; q < CP_CHUNKS; q++) {
+        if (kd[q] == KIND_NOP) continue;
+        const uint64_t i = i0 + 32 * q;
+        const uint32_t pos = bn + nn[q];
+        u.key[pos] = skey[i];
+        u.val[pos] = (uint8_t)(spay[i] & 0xFF);
+        u.kind[pos] = (uint8_t)kd[q];
+        u.seg[pos] = seg[i];
+        u.ip[pos] = bi + ni[q];
+    }
+    // the last CTA knows the totals: list length, inserts, the end of ip
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        const uint32_t nu = (uint32_t)all, nin = (uint32_t)(all >> 32);
+        st->n_u = nu;
+        st->n_ins = nin;
+        st->n_del = nu - nin;
+        u.ip[nu] = nin;
+    }
 }
 
 // ------------------------------------------------------------------ relocate / pending
@@ -2494,7 +2549,7 @@ void launch_compact(const uint64_t *k0, const uint16_t *p0, const uint64_t *k1, 
                     const uint32_t *sup, UpdList u, DevStatus *st, cudaStream_t s) {
     ProfScope ps_("compact", s);
     const uint32_t nb = (n + TPB - 1) / TPB;
-    launch_pdl(k_compact, dim3(nb), dim3(TPB), 0, s, k0, p0, k1, p1, mask, kind, seg, n, blk_nn, blk_ins, sup, u, st);
+    launch_pdl(k_compact, dim3((nb + CP_CHUNKS - 1) / CP_CHUNKS), dim3(TPB), 0, s, k0, p0, k1, p1, mask, kind, seg, n, blk_nn, blk_ins, sup, u, st);
     note_launch();
 }
 
@@ -2525,6 +2580,9 @@ void launch_plan(const UpdList u, uint32_t n_cap, const uint8_t *cnt, const uint
     uint32_t nb = (n_cap + TPB - 1) / TPB;
     if (!nb) return;
     Absorbed ab{nullptr, nullptr, 0};
+    // the CTAs loop over chunks of the list; with one each, the plan of a bulk
+    // load of 16.8M keys, which ends at once, took 190 us instead of 53
+    nb = std::min<uint32_t>(nb, 152 * 16);
     if (part) {
         nb = std::min<uint32_t>(nb, 152 * 4);
         ab = Absorbed{part->absbits, part->bwin, 2u << (H - part->L)};
