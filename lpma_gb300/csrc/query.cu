@@ -559,11 +559,13 @@ __global__ void k_zero_f64(double *p) { *p = 0.0; }
 // threads added in shared memory; a chunk adds at most 1,024 sums to acc.
 //
 // The push form (k_pr_push) makes one f64 atomic an edge: 276-300 us an
-// iteration on a scale-20 graph (16.8M edges).  This form takes 124 after
-// 356 for the layout; bound by the random 8-byte reads of contrib (one a
-// stored edge, out of L2: 5.4 TB/s of 32-byte sectors).
-constexpr uint32_t PR_LOW = 10, PR_BIN = 1u << PR_LOW, PR_MAX_BINS = 4096, PR_CHUNK = 16384;
-constexpr uint32_t PR_SORT_TPB = 1024, PR_PULL_TPB = 512, PR_EPT = PR_CHUNK / PR_PULL_TPB;
+// iteration on a scale-20 graph (16.8M edges).  This form takes 104 (89 of
+// them the sums) after 342 for the layout; bound by the random 8-byte reads
+// of contrib (one a stored edge, out of L2: 5.5 TB/s of 32-byte sectors) and
+// the FP64 adds.  Chunks of 8,192 edges by 256 threads: 97 with 16,384 by
+// 512, whose CTAs wait longer for their last warp.
+constexpr uint32_t PR_LOW = 10, PR_BIN = 1u << PR_LOW, PR_MAX_BINS = 4096, PR_CHUNK = 8192;
+constexpr uint32_t PR_SORT_TPB = 1024, PR_PULL_TPB = 256, PR_EPT = PR_CHUNK / PR_PULL_TPB;
 constexpr uint32_t PR_TILE_SEGS = 512;  // segments a CTA counts or places
 
 // the edges of segment s: f(src, dst) on each of the group's lanes
@@ -762,35 +764,45 @@ __global__ void __launch_bounds__(TPB) k_pr_deg(const uint32_t *__restrict__ P, 
 
 // rank (1/V when init, else from acc and *dangling), contrib = rank / deg,
 // the next dangling sum; clears acc and the dangling word after that
+// (base = (1 - alpha) / V, first = 1 / V).
+//
+// Bound by the FP64 pipes, which take two lanes a clock: six operations a
+// vertex.  So no thread divides (three quotients a thread took 20 of the
+// 28 us of a step over 1M vertices), and zero sums are not added up.
 __global__ void __launch_bounds__(TPB) k_pr_step(bool init, double *rank, double *acc, const double *__restrict__ inv,
-                                                 const uint32_t *__restrict__ deg, uint32_t V, double alpha,
-                                                 const double *__restrict__ dangling, double *next, double *after,
-                                                 double *contrib) {
-    __shared__ double ws[TPB / 32];
-    const double base = (1.0 - alpha) / (double)V, dv = init ? 0.0 : *dangling / (double)V, first = 1.0 / (double)V;
+                                                 const uint32_t *__restrict__ deg, uint32_t V, double alpha, double base,
+                                                 double first, const double *__restrict__ dangling, double *next,
+                                                 double *after, double *contrib) {
+    __shared__ double ws[TPB / 32], s_dv;
+    if (threadIdx.x == 0) s_dv = init ? 0.0 : *dangling / (double)V;
+    __syncthreads();
+    const double dv = s_dv;
     double d = 0;
     for (uint64_t v = blockIdx.x * (uint64_t)TPB + threadIdx.x; v < V; v += gridDim.x * (uint64_t)TPB) {
         const double r = init ? first : base + alpha * (acc[v] + dv);
         rank[v] = r;
         acc[v] = 0.0;
         const double i = inv[v];
-        if (i == 0.0) {
+        const uint32_t n = deg[v];
+        if (n == 0) {
             contrib[v] = 0.0;
             d += r;
         } else {
             // rank / deg from the rounded reciprocal: one correction step
             // gives the quotient's rounding
             const double q = r * i;
-            contrib[v] = fma(fma(-q, (double)deg[v], r), i, q);
+            contrib[v] = fma(fma(-q, (double)n, r), i, q);
         }
     }
+    if (__any_sync(0xffffffffu, __double_as_longlong(d) != 0))
 #pragma unroll
-    for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = d;
     __syncthreads();
     if (threadIdx.x == 0) {
         double t = 0;
-        for (int i = 0; i < TPB / 32; i++) t += ws[i];
+        for (int i = 0; i < TPB / 32; i++)
+            if (__double_as_longlong(ws[i]) != 0) t += ws[i];
         if (t != 0.0) atomicAdd(next, t);
         if (blockIdx.x == 0) *after = 0.0;
     }
@@ -918,7 +930,7 @@ void launch_pr_pull(uint32_t it, const PrLayout &l, const uint32_t *words, uint3
         note_launch();
     }
     k_pr_step<<<grid_for(V, TPB, 152 * 8), TPB, 0, s>>>(it == 0, rank, acc, inv, deg, V, alpha,
-                                                        dangling + it % 3, dangling + (it + 1) % 3,
+                                                        (1.0 - alpha) / (double)V, 1.0 / (double)V, dangling + it % 3, dangling + (it + 1) % 3,
                                                         dangling + (it + 2) % 3, contrib);
     note_launch();
 }
