@@ -298,7 +298,7 @@ LPMA_API lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *grap
                                          size_t n, lpma_stream_t stream, LpmaStats *stats, lpma_status_t *status);
 
 /* ---- autotuner: the batch-sort algorithm per batch-size bucket ----
- * Batches of 256 to 2^21 keys on trees of height 9 and more take the
+ * Batches of 256 to 2^21 keys, no more than are stored, on trees of height 9 and more take the
  * partitioned front, which does not sort the whole batch, unless they
  * crowd into one of its buckets; lpma_tune_set with a tier other than 0
  * keeps the batches of its entry off it.  The sorted front sorts each batch

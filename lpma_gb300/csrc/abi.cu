@@ -786,10 +786,12 @@ lpma_status_t enqueue_part(LpmaHandle *h, cudaStream_t s, const PartArgs &pa, si
 }
 
 // The partitioned front's plan for a batch (L = 0: the sorted front): not
-// for the engine's own sentinels, a sort tier set by the caller, or a handle
-// whose buckets overflowed lately.
+// for the engine's own sentinels, a sort tier set by the caller, a handle
+// whose buckets overflowed lately, or a batch of more keys than are stored,
+// whose spread the tree does not know (the buckets of a skewed first load
+// overflow).
 PartPlan plan_part(LpmaHandle *h, size_t n, bool internal) {
-    if (internal || h->part_skip || sort_tier_forced((uint32_t)n, h->sort)) return PartPlan{};
+    if (internal || h->part_skip || n > h->total || sort_tier_forced((uint32_t)n, h->sort)) return PartPlan{};
     return part_plan(n, h->H);
 }
 

@@ -1004,7 +1004,10 @@ lpma_status_t exec_bigs(GpmaState *g, const Window *wbig, uint32_t n_big, const 
 // 128 to 256; a bucket has room for 3.5 times the average.
 void gpma_part_plan(const GpmaState *g, uint64_t n, uint32_t *L, uint32_t *cap) {
     *L = 0;
-    if (n > GP_MAX || g->h < 6) return;
+    // (not a batch of more keys than are stored, whose spread the array does
+    // not know: the buckets of a skewed first load overflow, 400 us in vain
+    // before the sort of 1M keys)
+    if (n > GP_MAX || n > g->live_total || g->h < 6) return;
     uint32_t l = 1;
     while (l < std::min(GP_L_MAX, g->h - 1) && (n >> (l + 1)) >= (l < 7 ? 32 : 128)) l++;
     const uint64_t avg = (n + (1u << l) - 1) >> l;
