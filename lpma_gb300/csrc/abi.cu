@@ -24,6 +24,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -69,6 +70,13 @@ struct FrontGraph {
     cudaGraphExec_t exec;
     cudaGraphNode_t pack;
     cudaKernelNodeParams pack_params;
+};
+
+struct BatchEvent {
+    cudaEvent_t ev = nullptr;
+    ~BatchEvent() {
+        if (ev) cudaEventDestroy(ev);
+    }
 };
 
 }  // namespace
@@ -125,6 +133,8 @@ struct LpmaHandle {
     // flight, on the call's stream: lpma_destroy waits for it, not the device
     cudaEvent_t done_ev = nullptr;
     bool done_recorded = false;
+    std::shared_ptr<BatchEvent> batch_done;  // the same of its last batched update, one event for all graphs
+    uint64_t batch_call = 0;                 // the batched update that it was last part of
     // LPMA_FLAG_GPMA: the flat array of gpma.cuh (gpma.cu) instead of the
     // leveled tree; the leveled fields above stay unused
     GpmaState *gp = nullptr;
@@ -999,10 +1009,11 @@ lpma_status_t wait_front(LpmaHandle *h, cudaStream_t) {
 // the graphs of a batched update.  small_done: the first loop's single / 4 /
 // 32-segment executors already ran (in lpma_update's front, guarded, or in
 // the shared launches of a batched update).  front_counts: so is the recount
-// that a call with an expiry threshold ends with.
+// that a call with an expiry threshold ends with.  batch: the event that the
+// caller records once behind the last of many graphs' work.
 lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t thres, bool thres_active,
                             cudaStream_t s, LpmaStats &st, LpmaStats *out, bool small_done = false,
-                            bool front_counts = false) {
+                            bool front_counts = false, const std::shared_ptr<BatchEvent> *batch = nullptr) {
     // a sort that gave up a bounded wait turned the front into a no-op:
     // nothing changed, so the handle stays usable
     if (rs == LPMA_ERR_TIMEOUT && h->hst->sticky == 0) return rs;
@@ -1121,7 +1132,10 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
     st.h2d_bytes = h->h2d;
     st.d2h_bytes = h->d2h;
     if (out) *out = st;
-    mark_done(h, s);
+    if (batch)
+        h->batch_done = *batch;  // an event a graph took half a microsecond
+    else
+        mark_done(h, s);
     return LPMA_OK;
 }
 
@@ -1272,6 +1286,7 @@ struct LpmaBatcher {
     cudaStream_t side = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     bool pending = false;
+    std::shared_ptr<BatchEvent> all;        // after the shared graphs' last work of a call
     BatchWorkers *workers = nullptr;
 };
 
@@ -1365,6 +1380,7 @@ lpma_status_t lpma_destroy(LpmaHandle *h) {
     // then every buffer goes back to the stream-ordered pool without a
     // device-wide synchronisation, so other handles' streams keep running
     if (h->done_recorded) cudaEventSynchronize(h->done_ev);
+    if (h->batch_done) cudaEventSynchronize(h->batch_done->ev);
     for (cudaStream_t st : {h->side_stream, h->cap_stream, h->copy_stream})
         if (st) cudaStreamSynchronize(st);
     for (FrontGraph &f : h->graphs) {
@@ -1940,8 +1956,8 @@ lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *graphs, const
     std::vector<lpma_status_t> res(n, LPMA_OK);
     std::vector<LpmaStats> sts(n);
     std::vector<size_t> forest, plain;
-    std::vector<LpmaHandle *> seen;
-    seen.reserve(n);
+    static std::atomic<uint64_t> g_calls{0};
+    const uint64_t call = ++g_calls;
     for (size_t i = 0; i < n; i++) {
         LpmaHandle *h = graphs[i];
         const LpmaBatch &it = items[i];
@@ -1950,11 +1966,11 @@ lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *graphs, const
             res[i] = LPMA_ERR_INVALID_ARGUMENT;
             continue;
         }
-        if (std::find(seen.begin(), seen.end(), h) != seen.end()) {  // one batch per graph per call
+        if (h->batch_call == call) {  // one batch per graph per call
             res[i] = LPMA_ERR_INVALID_ARGUMENT;
             continue;
         }
-        seen.push_back(h);
+        h->batch_call = call;
         if (h->sticky != LPMA_OK) {
             res[i] = h->sticky;
             continue;
@@ -2105,6 +2121,11 @@ lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *graphs, const
         // shared executors (host work, maybe an eager level-up), then the
         // rest, whose paths wait on the device, on several host threads
         std::vector<uint32_t> rest;
+        if (GS && !b->all) {
+            auto ev = std::make_shared<BatchEvent>();
+            CK(cudaEventCreateWithFlags(&ev->ev, cudaEventDisableTiming));
+            b->all = std::move(ev);
+        }
         auto finish = [&](uint32_t k, cudaStream_t st) {
             const size_t i = forest[k];
             LpmaHandle *h = graphs[i];
@@ -2116,7 +2137,7 @@ lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *graphs, const
             h->front_sort_wide = false;  // the shared tile-merge sort
             h->front_part = false;
             res[i] = finish_update(h, rs, items[i].n_ins + items[i].n_del, 0, false, st, sts[i], &sts[i],
-                                   shared[k] != 0);
+                                   shared[k] != 0, false, shared[k] ? &b->all : nullptr);
         };
         for (uint32_t k = 0; k < G; k++) {
             if (shared[k])
@@ -2124,6 +2145,7 @@ lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *graphs, const
             else
                 rest.push_back(k);
         }
+        if (GS) CK(cudaEventRecord(b->all->ev, s));
         if (rest.size() > 1 && !prof_enabled()) {
             if (!b->workers) {
                 b->workers = new BatchWorkers();

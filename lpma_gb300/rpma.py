@@ -8,6 +8,7 @@ tensors (device path, ``lpma_update``) or numpy arrays (host path,
 implementation behind this module.
 """
 import ctypes
+from array import array
 
 import numpy as np
 
@@ -88,17 +89,17 @@ def _is_cuda_tensor(x):
 
 
 _SAME_BITS = {"uint64": ("torch.uint64", "torch.int64"), "uint8": ("torch.uint8", "torch.int8")}
-_OK_DTYPES = {}
+_OK_DTYPES = {"uint64": set(), "uint8": set()}  # dtypes met so far that are taken
 
 
 def _dev(x, dtype_name):
     if x is None:
         return None, 0
-    ok = _OK_DTYPES.get((x.dtype, dtype_name))
-    if ok is None:
-        ok = _OK_DTYPES[(x.dtype, dtype_name)] = str(x.dtype) in _SAME_BITS[dtype_name]
-    if not ok:
-        raise TypeError("expected a torch.%s tensor, got %s" % (dtype_name, x.dtype))
+    ok = _OK_DTYPES[dtype_name]
+    if x.dtype not in ok:
+        if str(x.dtype) not in _SAME_BITS[dtype_name]:
+            raise TypeError("expected a torch.%s tensor, got %s" % (dtype_name, x.dtype))
+        ok.add(x.dtype)
     if not x.is_contiguous():
         raise ValueError("device inputs must be contiguous")
     return x.data_ptr(), x.numel()
@@ -401,25 +402,23 @@ class Batcher:
         ins_vals, dels, thres (or an (ins, dels) pair).  Returns (stats,
         statuses), one entry per graph."""
         n = len(graphs)
-        items = (_abi.LpmaBatch * n)()
-        hs = (ctypes.c_void_p * n)()
-        keep = []
-        for i, (g, b) in enumerate(zip(graphs, batches)):
+        # LpmaBatch records as six 64-bit words each: 256 graphs took 528 us a
+        # struct field at a time, 415 so (240 of them in the tensors' own calls)
+        words = array("Q")
+        for _, b in zip(graphs, batches):
             if not isinstance(b, dict):
                 b = {"ins": b[0], "dels": b[1]}
-            hs[i] = g._h.value
-            it = items[i]
-            if b.get("ins") is not None:
-                it.ins, it.n_ins = _dev(b["ins"], "uint64")
-            if b.get("ins_vals") is not None:
-                it.ins_vals = _dev(b["ins_vals"], "uint8")[0]
-            if b.get("dels") is not None:
-                it.dels, it.n_del = _dev(b["dels"], "uint64")
-            it.thres = int(b.get("thres", 0))
-            keep.append(b)
+            ins, vals, dels = b.get("ins"), b.get("ins_vals"), b.get("dels")
+            pi, ni = _dev(ins, "uint64") if ins is not None else (0, 0)
+            pd, nd = _dev(dels, "uint64") if dels is not None else (0, 0)
+            words.extend((pi, _dev(vals, "uint8")[0] if vals is not None else 0, ni, pd, nd,
+                          int(b.get("thres", 0)) & 0xFFFFFFFF))
+        words.extend([0] * (6 * n - len(words)))
+        hs = array("Q", [g._h.value or 0 for g in graphs])
         stats = (LpmaStats * n)()
         status = (ctypes.c_int * n)()
-        rc = self._L.lpma_update_batch(self._b, hs, items, n, _stream_ptr(stream), stats, status)
+        rc = self._L.lpma_update_batch(self._b, hs.buffer_info()[0], words.buffer_info()[0], n, _stream_ptr(stream), stats,
+                                       status)
         if raise_on_error:
             check(rc, "lpma_update_batch")
         return list(stats), list(status)
