@@ -532,13 +532,16 @@ def roofline(res, B, peak, peak_kind, name=None):
     cnt, ms = prof[name]
     pst = res["pstats"]
     # algorithmic bytes per launch of the dominant kernel
-    if name == "exec_single":
+    if name in ("exec_single", "bucket"):  # the buckets order and locate their keys as well
         units = sum(32 * s["windows_single"] for s in pst) / cnt
         per_unit, unit_name = 18, "window slot (8 B key + 1 B value, read and written)"
     elif name == "exec_small":
         units = sum(s["slots_small"] - 32 * s["windows_single"] for s in pst) / cnt
         per_unit, unit_name = 18, "window slot (8 B key + 1 B value, read and written)"
-    elif name == "exec_tiles":
+    elif name == "part":
+        units = B
+        per_unit, unit_name = 24, "key (8 B read, 16 B entry written)"
+    elif name in ("exec_tiles", "respread"):
         units = sum(s["slots_rewritten"] - s["slots_small"] for s in pst) / cnt
         per_unit, unit_name = 18, "window slot (8 B key + 1 B value, read and written)"
     elif name == "sort_coop":
@@ -577,18 +580,20 @@ def roofline(res, B, peak, peak_kind, name=None):
 
 
 REBALANCE_CLASSES = (
-    ("single", ("exec_single",)),
+    ("single", ("exec_single", "bucket")),
     ("small", ("exec_small", "exec_small4", "exec_small32")),
-    ("big", ("exec_gather", "exec_spread", "seg_counts", "seg_q", "scan")),
+    ("big", ("exec_gather", "exec_spread", "seg_counts", "seg_q", "scan", "respread", "respread_tiles")),
 )
 
 
 def rebalance_roofline(res, peak, peak_kind):
     """Window rewrites of the profiled steps, by executor class and in total:
     18 B per rewritten slot (8 B key + 1 B value, read and written) over the
-    summed device time of the class's kernels.  single: one-segment windows;
-    small: 2..32 segments; big: larger windows, the root and rebuilds
-    (gather / spread with their tile preparation)."""
+    summed device time of the class's kernels.  single: one-segment windows
+    (with the partitioned front's locating and ordering, which the same
+    kernel does); small: 2..32 segments; big: larger windows, the root and
+    rebuilds (gather / spread with their tile preparation, or the one-pass
+    respread)."""
     prof, pst = res["prof"], res["pstats"]
     if not prof or not pst:
         return None
