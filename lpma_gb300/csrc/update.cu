@@ -1833,8 +1833,10 @@ __global__ void __launch_bounds__(TPB) k_ts_down(const uint8_t *__restrict__ cnt
 // Windows larger than 32 segments (root, level >= 6, rebuild) run in two
 // fully parallel phases.  Gather: one 8-lane group per source segment merges
 // its kept slots with the inserts located into it and writes them, in
-// window rank order, to a contiguous sequence M (the alternate buffer) at
-// PQ[s] + rank.  Spread: one 8-lane group per destination segment takes its
+// window rank order, to a sequence M (the alternate buffer) that starts at
+// its own first slot: the window's share of PQ (which counts the updates of
+// windows that executed in the same loop a second time, so its absolute
+// values do not serve) + rank.  Spread: one 8-lane group per destination segment takes its
 // items [first_rank(k), first_rank(k+1)) from M.  Every source slot is read
 // before any destination slot is written (two launches), so the windows are
 // rewritten in place.
@@ -1881,7 +1883,7 @@ __global__ void __launch_bounds__(GT_TPB) k_gather(const TileJob *__restrict__ j
             }
             us = US[s];
             ue = US[s + 1];
-            base = PQ[s];
+            base = 32ull * J.sa + (PQ[s] - PQ[J.sa]);
         }
         const uint32_t nl = __popc(kmask);
         uint32_t incl = nl;
@@ -2005,7 +2007,7 @@ __global__ void __launch_bounds__(TPB) k_gather_ins(const TileJob *__restrict__ 
             for (uint32_t t = 0; t < pos; t++)
                 expired_below += (sv[t] != VAL_TOMB && (sk[t] & TIME_MASK) < (uint64_t)thres) ? 1u : 0u;
         }
-        const uint64_t r = (uint64_t)PQ[s] + ri + (pos - tomb_below - expired_below);
+        const uint64_t r = 32ull * jobs[L].sa + (PQ[s] - PQ[jobs[L].sa]) + ri + (pos - tomb_below - expired_below);
         if (r < m_cap) {
             Mk[r] = y;
             Mv[r] = u.val[x];
@@ -2027,8 +2029,8 @@ __global__ void __launch_bounds__(GT_TPB) k_spread(const TileJob *__restrict__ j
         const uint64_t inv = ~0ull / J.df;  // the same for every thread of the tile
         const uint64_t k = 32ull * (tile - J.dtile0) + grp;
         if (k >= J.df) continue;
-        const uint64_t mb = PQ[J.sa];
-        if (k == 0 && gl == 0 && PQ[J.sa + J.sf] - mb != J.m) {  // the gather must account for m items
+        const uint64_t mb = 32ull * J.sa;
+        if (k == 0 && gl == 0 && PQ[J.sa + J.sf] - PQ[J.sa] != J.m) {  // the gather must account for m items
             atomicOr(&st->sticky, ERR_INTERNAL);
             atomicCAS(&st->sticky_site, 0u, 2u);
         }
