@@ -850,9 +850,12 @@ lpma_status_t run_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, cons
     h->hinit->total_items = h->total;
     h->hinit->thres = thres;
     h->hinit->seq++;
-    const PartPlan pp = plan_part(h, n, internal);
+    PartPlan pp = plan_part(h, n, internal);
+    if (pp.L && ensure_part(h, pp, s) != LPMA_OK) {  // no room for the buckets: the sorted front needs none
+        cudaGetLastError();
+        pp = PartPlan{};
+    }
     h->front_part = pp.L != 0;
-    if (pp.L) CKS(ensure_part(h, pp, s));
     const PartArgs pa{ins, ins_vals, del, (uint32_t)n_ins, (uint32_t)n_del, h->V, thres, h->cfg.key_format, pp.L, pp.cap,
                       pp.ipt, h->c.fl, h->part_ent, h->part_ctl, h->dst};
     auto enqueue = [&](cudaStream_t st) {
@@ -1837,7 +1840,10 @@ lpma_status_t lpma_pagerank(LpmaHandle *h, double alpha, uint32_t iterations, do
         CK(dalloc(&h->pr_dangling, 3));
     }
     const Geo g{h->c.keys, h->c.vals, h->H};
-    if (pagerank_pulls(h->total - h->V, iterations)) {
+    // (a captured call allocates nothing and pushes)
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &cs));
+    if (cs == cudaStreamCaptureStatusNone && pagerank_pulls(h->total - h->V, iterations)) {
         // the edges by destination and the reciprocal degrees, for this call
         PrLayout l;
         const uint64_t words = pr_words(h->V, h->total - h->V, &l);
