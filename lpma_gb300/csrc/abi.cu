@@ -1849,16 +1849,16 @@ lpma_status_t lpma_pagerank(LpmaHandle *h, double alpha, uint32_t iterations, do
         const uint64_t words = pr_words(h->V, h->total - h->V, &l);
         const size_t at = (words * 4 + 255) & ~size_t(255);
         void *mem = nullptr;
-        const cudaError_t e = pool_alloc(&mem, at + sizeof(double) * h->V, s);
+        const cudaError_t e = pool_alloc(&mem, at + sizeof(double2) * h->V, s);
         if (e == cudaSuccess) {
             uint32_t *w = static_cast<uint32_t *>(mem);
-            double *inv = reinterpret_cast<double *>(static_cast<char *>(mem) + at);
+            double2 *inv = reinterpret_cast<double2 *>(static_cast<char *>(mem) + at);
             const uint64_t nseg = nseg_of(h->H);
             cudaError_t x = scan_u8_to_u32(h->c.cnt, h->c.segP, (uint32_t)nseg, h->c.segP + nseg, h->c.scan_tmp, s);
-            if (!x) x = launch_pr_layout(g, h->c.cnt, h->c.segP, h->sent, h->V, l, w, inv, h->pr_deg, s);
+            if (!x) x = launch_pr_layout(g, h->c.cnt, h->c.segP, h->sent, h->V, l, w, inv, s);
             if (!x) x = cudaMemsetAsync(h->pr_dangling, 0, 3 * sizeof(double), s);
             for (uint32_t it = 0; it <= iterations && !x; it++)
-                launch_pr_pull(it, l, w, h->V, alpha, inv, h->pr_deg, d_rank, h->pr_contrib, h->pr_acc, h->pr_dangling,
+                launch_pr_pull(it, l, w, h->V, alpha, inv, d_rank, h->pr_contrib, h->pr_acc, h->pr_dangling,
                                s);
             if (!x) x = cudaGetLastError();
             const cudaError_t f = cudaFreeAsync(mem, s);

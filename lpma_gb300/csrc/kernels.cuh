@@ -255,9 +255,9 @@ struct PrLayout {
 };
 size_t pr_words(uint32_t V, uint64_t edges, PrLayout *l);
 cudaError_t launch_pr_layout(Geo g, const uint8_t *cnt, const uint32_t *P, const uint32_t *sent, uint32_t V,
-                             const PrLayout &l, uint32_t *words, double *inv, uint32_t *deg, cudaStream_t s);
-void launch_pr_pull(uint32_t it, const PrLayout &l, const uint32_t *words, uint32_t V, double alpha, const double *inv,
-                    const uint32_t *deg, double *rank, double *contrib, double *acc, double *dangling,
+                             const PrLayout &l, uint32_t *words, double2 *inv, cudaStream_t s);
+void launch_pr_pull(uint32_t it, const PrLayout &l, const uint32_t *words, uint32_t V, double alpha, const double2 *inv,
+                    double *rank, double *contrib, double *acc, double *dangling,
                     cudaStream_t s);
 void launch_pr_iteration(Geo g, const uint8_t *cnt, const uint32_t *deg, uint32_t V, double alpha, double *rank,
                          double *contrib, double *acc, double *dangling, cudaStream_t s);

@@ -559,7 +559,7 @@ __global__ void k_zero_f64(double *p) { *p = 0.0; }
 // threads added in shared memory; a chunk adds at most 1,024 sums to acc.
 //
 // The push form (k_pr_push) makes one f64 atomic an edge: 276-300 us an
-// iteration on a scale-20 graph (16.8M edges).  This form takes 104 (89 of
+// iteration on a scale-20 graph (16.8M edges).  This form takes 102 (86 of
 // them the sums) after 342 for the layout; bound by the random 8-byte reads
 // of contrib (one a stored edge, out of L2: 5.5 TB/s of 32-byte sectors) and
 // the FP64 adds.  Chunks of 8,192 edges by 256 threads: 97 with 16,384 by
@@ -751,14 +751,14 @@ __global__ void __launch_bounds__(PR_PULL_TPB) k_pr_pull(const uint4 *__restrict
 }
 
 // out-degrees from the slot ranks of the sentinels (P: exclusive prefix of
-// the segment counts), and their reciprocals
+// the segment counts): their reciprocals, and they themselves
 __global__ void __launch_bounds__(TPB) k_pr_deg(const uint32_t *__restrict__ P, const uint32_t *__restrict__ sent,
-                                                uint32_t H, uint32_t V, double *inv, uint32_t *deg) {
+                                                uint32_t H, uint32_t V, double2 *inv) {
     for (uint64_t v = blockIdx.x * (uint64_t)TPB + threadIdx.x; v < V; v += gridDim.x * (uint64_t)TPB) {
         const uint64_t p1 = linear_slot(sent[v], H), p0 = v ? linear_slot(sent[v - 1], H) : 0;
         const uint32_t r1 = P[p1 >> 5] + (uint32_t)(p1 & 31), r0 = v ? P[p0 >> 5] + (uint32_t)(p0 & 31) + 1 : 0u;
-        deg[v] = r1 - r0;
-        inv[v] = r1 > r0 ? 1.0 / (double)(r1 - r0) : 0.0;
+        const double n = (double)(r1 - r0);
+        inv[v] = r1 > r0 ? make_double2(1.0 / n, n) : make_double2(0.0, 0.0);
     }
 }
 
@@ -766,12 +766,11 @@ __global__ void __launch_bounds__(TPB) k_pr_deg(const uint32_t *__restrict__ P, 
 // the next dangling sum; clears acc and the dangling word after that
 // (base = (1 - alpha) / V, first = 1 / V).
 //
-// Bound by the FP64 pipes, which take two lanes a clock: six operations a
-// vertex.  So no thread divides (three quotients a thread took 20 of the
+// Bound by the FP64 pipes, which take two lanes a clock: five operations a
+// vertex, the degree being stored as a double beside its reciprocal.  So no thread divides (three quotients a thread took 20 of the
 // 28 us of a step over 1M vertices), and zero sums are not added up.
-__global__ void __launch_bounds__(TPB) k_pr_step(bool init, double *rank, double *acc, const double *__restrict__ inv,
-                                                 const uint32_t *__restrict__ deg, uint32_t V, double alpha, double base,
-                                                 double first, const double *__restrict__ dangling, double *next,
+__global__ void __launch_bounds__(TPB) k_pr_step(bool init, double *rank, double *acc, const double2 *__restrict__ inv,
+                                                 uint32_t V, double alpha, double base, double first, const double *__restrict__ dangling, double *next,
                                                  double *after, double *contrib) {
     __shared__ double ws[TPB / 32], s_dv;
     if (threadIdx.x == 0) s_dv = init ? 0.0 : *dangling / (double)V;
@@ -782,16 +781,15 @@ __global__ void __launch_bounds__(TPB) k_pr_step(bool init, double *rank, double
         const double r = init ? first : base + alpha * (acc[v] + dv);
         rank[v] = r;
         acc[v] = 0.0;
-        const double i = inv[v];
-        const uint32_t n = deg[v];
-        if (n == 0) {
+        const double2 i = inv[v];
+        if (__double_as_longlong(i.y) == 0) {
             contrib[v] = 0.0;
             d += r;
         } else {
             // rank / deg from the rounded reciprocal: one correction step
             // gives the quotient's rounding
-            const double q = r * i;
-            contrib[v] = fma(fma(-q, (double)n, r), i, q);
+            const double q = r * i.x;
+            contrib[v] = fma(fma(-q, i.y, r), i.x, q);
         }
     }
     if (__any_sync(0xffffffffu, __double_as_longlong(d) != 0))
@@ -901,7 +899,7 @@ size_t pr_words(uint32_t V, uint64_t edges, PrLayout *l) {
 }
 
 cudaError_t launch_pr_layout(Geo g, const uint8_t *cnt, const uint32_t *P, const uint32_t *sent, uint32_t V,
-                             const PrLayout &l, uint32_t *words, double *inv, uint32_t *deg, cudaStream_t s) {
+                             const PrLayout &l, uint32_t *words, double2 *inv, cudaStream_t s) {
     cudaError_t e = cudaFuncSetAttribute(k_pr_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)((2 * PR_CHUNK + PR_BIN + 32) * 4));
     if (e != cudaSuccess) return e;
@@ -914,13 +912,13 @@ cudaError_t launch_pr_layout(Geo g, const uint8_t *cnt, const uint32_t *P, const
     k_pr_table<<<1, 1024, 0, s>>>(l.nbins, bins, chunks, n_chunks);
     k_pr_place<<<tiles, TPB, 0, s>>>(g, cnt, l.nbins, bins, edges, l.cap);
     k_pr_sort<<<l.max_chunks, PR_SORT_TPB, (2 * PR_CHUNK + PR_BIN + 32) * 4, s>>>(chunks, n_chunks, edges);
-    k_pr_deg<<<grid_for(V, TPB, 152 * 8), TPB, 0, s>>>(P, sent, g.H, V, inv, deg);
+    k_pr_deg<<<grid_for(V, TPB, 152 * 8), TPB, 0, s>>>(P, sent, g.H, V, inv);
     note_launch(5);
     return cudaGetLastError();
 }
 
-void launch_pr_pull(uint32_t it, const PrLayout &l, const uint32_t *words, uint32_t V, double alpha, const double *inv,
-                    const uint32_t *deg, double *rank, double *contrib, double *acc, double *dangling,
+void launch_pr_pull(uint32_t it, const PrLayout &l, const uint32_t *words, uint32_t V, double alpha, const double2 *inv,
+                    double *rank, double *contrib, double *acc, double *dangling,
                     cudaStream_t s) {
     ProfScope ps_("pagerank", s);
     const uint4 *chunks = reinterpret_cast<const uint4 *>(words);
@@ -929,7 +927,7 @@ void launch_pr_pull(uint32_t it, const PrLayout &l, const uint32_t *words, uint3
         k_pr_pull<<<l.max_chunks, PR_PULL_TPB, 0, s>>>(chunks, n_chunks, edges, contrib, acc, V);
         note_launch();
     }
-    k_pr_step<<<grid_for(V, TPB, 152 * 8), TPB, 0, s>>>(it == 0, rank, acc, inv, deg, V, alpha,
+    k_pr_step<<<grid_for(V, TPB, 152 * 8), TPB, 0, s>>>(it == 0, rank, acc, inv, V, alpha,
                                                         (1.0 - alpha) / (double)V, 1.0 / (double)V, dangling + it % 3, dangling + (it + 1) % 3,
                                                         dangling + (it + 2) % 3, contrib);
     note_launch();
