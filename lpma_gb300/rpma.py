@@ -405,10 +405,12 @@ class Batcher:
         # LpmaBatch records as six 64-bit words each: 256 graphs took 528 us a
         # struct field at a time, 415 so (240 of them in the tensors' own calls)
         words = array("Q")
+        keep = []  # the words hold addresses: an iterator's batches live in here until the call returns
         for _, b in zip(graphs, batches):
             if not isinstance(b, dict):
                 b = {"ins": b[0], "dels": b[1]}
             ins, vals, dels = b.get("ins"), b.get("ins_vals"), b.get("dels")
+            keep.append((ins, vals, dels))
             pi, ni = _dev(ins, "uint64") if ins is not None else (0, 0)
             pd, nd = _dev(dels, "uint64") if dels is not None else (0, 0)
             words.extend((pi, _dev(vals, "uint8")[0] if vals is not None else 0, ni, pd, nd,
