@@ -415,8 +415,10 @@ class Batcher:
             pd, nd = _dev(dels, "uint64") if dels is not None else (0, 0)
             words.extend((pi, _dev(vals, "uint8")[0] if vals is not None else 0, ni, pd, nd,
                           int(b.get("thres", 0)) & 0xFFFFFFFF))
+        # a graph without a batch is refused: it gets no handle
         words.extend([0] * (6 * n - len(words)))
-        hs = array("Q", [g._h.value or 0 for g in graphs])
+        hs = array("Q", [g._h.value or 0 for g, _ in zip(graphs, keep)])
+        hs.extend([0] * (n - len(hs)))
         stats = (LpmaStats * n)()
         status = (ctypes.c_int * n)()
         rc = self._L.lpma_update_batch(self._b, hs.buffer_info()[0], words.buffer_info()[0], n, _stream_ptr(stream), stats,

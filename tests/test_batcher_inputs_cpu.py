@@ -76,3 +76,17 @@ def test_batches_of_an_iterator_live_until_the_call_returns(batcher):
     assert batcher._L.items == [(0x1000 * (i + 1), 10 + i, 0x100000 * (i + 1), 3, 0) for i in range(6)]
     gc.collect()
     assert all(r() is None for r in watched)  # and no longer
+
+
+@pytest.mark.parametrize("n_batches", [0, 2, 3, 4])
+def test_graphs_without_a_batch_get_no_handle(batcher, n_batches):
+    """The library refuses a null handle (invalid argument), so a call with
+    fewer batches than graphs is refused for the graphs left over; batches
+    beyond the graphs are not looked at."""
+    batcher._L = FakeLib()
+    graphs = [FakeGraph(0x10 * (i + 1)) for i in range(3)]
+    batches = [(FakeTensor(0x1000 * (i + 1), i + 1), None) for i in range(n_batches)]
+    batcher.update(graphs, batches)
+    m = min(n_batches, 3)
+    assert batcher._L.handles == [0x10 * (i + 1) for i in range(m)] + [0] * (3 - m)
+    assert batcher._L.items == [(0x1000 * (i + 1), i + 1, None, 0, 0) for i in range(m)] + [(None, 0, None, 0, 0)] * (3 - m)
