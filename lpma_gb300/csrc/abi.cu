@@ -843,7 +843,8 @@ lpma_status_t run_front(LpmaHandle *h, cudaStream_t s, const uint64_t *ins, cons
     h->h2d += offsetof(DevStatus, sticky);
     h->d2h += sizeof(DevStatus);
     // the planner of this front sets it again (no GPU write to the mirror
-    // is pending: the last front's was waited for)
+    // is pending: the last front's was waited for, and so was its recount,
+    // unless the call was rejected, whose recount writes nothing)
     if (front_publishes(h)) __atomic_store_n(&h->hst->published, 0u, __ATOMIC_RELEASE);
     // the stored-key count reaches the planner through the status reset copy,
     // so that it is not a kernel argument of a cached graph
@@ -1017,11 +1018,17 @@ lpma_status_t wait_front(LpmaHandle *h, cudaStream_t) {
 lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t thres, bool thres_active,
                             cudaStream_t s, LpmaStats &st, LpmaStats *out, bool small_done = false,
                             bool front_counts = false, const std::shared_ptr<BatchEvent> *batch = nullptr) {
+    // what the front enqueued behind the status is still to be waited for
+    // by lpma_destroy, whatever the verdict
+    auto refused = [&](lpma_status_t why) {
+        mark_done(h, s);
+        return why;
+    };
     // a sort that gave up a bounded wait turned the front into a no-op:
     // nothing changed, so the handle stays usable
-    if (rs == LPMA_ERR_TIMEOUT && h->hst->sticky == 0) return rs;
-    if (rs != LPMA_OK) return h->sticky = rs;
-    if (h->hst->error & ERR_KEY) return LPMA_ERR_INVALID_KEY;
+    if (rs == LPMA_ERR_TIMEOUT && h->hst->sticky == 0) return refused(rs);
+    if (rs != LPMA_OK) return h->sticky = refused(rs);
+    if (h->hst->error & ERR_KEY) return refused(LPMA_ERR_INVALID_KEY);
     {
         // the digit passes the sort made: one per differing byte, or with
         // 9-bit digits one per window (the greedy plan of the sort itself)
@@ -1113,13 +1120,13 @@ lpma_status_t finish_update(LpmaHandle *h, lpma_status_t rs, size_t n, uint32_t 
             r = rebuild(h, hh, h->u, (uint32_t)n, (uint64_t)live_after, thres, thres_active, s, &st);
         }
     }
-    if (r != LPMA_OK) return h->sticky = r;
+    if (r != LPMA_OK) return h->sticky = refused(r);
     if (thres_active && front_counts && !front_ovf && !front_big) {
         // recounted behind the front's executors, which did everything
         CK(wait_published(h, true, s));
         h->d2h += 16;
         if (h->hst->sticky & (ERR_TIMEOUT | ERR_INTERNAL))
-            return h->sticky = (h->hst->sticky & ERR_TIMEOUT) ? LPMA_ERR_TIMEOUT : LPMA_ERR_INTERNAL;
+            return h->sticky = refused((h->hst->sticky & ERR_TIMEOUT) ? LPMA_ERR_TIMEOUT : LPMA_ERR_INTERNAL);
     } else if (thres_active) {
         // executed windows dropped expired keys: recount what is stored
         CK(cudaMemsetAsync(&h->dst->cnt_total, 0, 8, s));

@@ -2475,10 +2475,12 @@ __global__ void __launch_bounds__(TPB) k_check_empty_level(const uint8_t *__rest
 
 // Stored keys after a call with an expiry threshold.  pub: the last CTA puts
 // the sum and the sticky words into the host's mirror and then sets its
-// `counted` word to the call's number (an earlier call may have returned,
-// rejected, before its recount).
+// `counted` word to the call's number.  After a rejected call or one whose
+// sort gave up, which returns without waiting for its recount, and after a
+// bucket overflow nothing is counted or written.
 __global__ void __launch_bounds__(TPB) k_sum_cnt(const uint8_t *__restrict__ cnt, uint64_t nseg, DevStatus *st,
                                                  DevStatus *pub) {
+    if (st->error | st->part_ovf) return;
     uint32_t acc = 0;
     const uint64_t whole = nseg / 16;
     for (uint64_t i = blockIdx.x * (uint64_t)TPB + threadIdx.x; i < whole; i += gridDim.x * (uint64_t)TPB) {
