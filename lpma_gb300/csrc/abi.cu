@@ -33,6 +33,7 @@
 #include "kernels.cuh"
 #include "lpma.h"
 #include "prims.cuh"
+#include "spare_ring.h"
 
 using namespace lpma;
 
@@ -133,7 +134,7 @@ struct LpmaHandle {
     // flight, on the call's stream: lpma_destroy waits for it, not the device
     cudaEvent_t done_ev = nullptr;
     bool done_recorded = false;
-    std::shared_ptr<BatchEvent> batch_done;  // the same of its last batched update, one event for all graphs
+    std::shared_ptr<BatchEvent> batch_done;  // the same of its last batched update, one event for that call's graphs
     uint64_t batch_call = 0;                 // the batched update that it was last part of
     // LPMA_FLAG_GPMA: the flat array of gpma.cuh (gpma.cu) instead of the
     // leveled tree; the leveled fields above stay unused
@@ -1296,7 +1297,9 @@ struct LpmaBatcher {
     cudaStream_t side = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     bool pending = false;
-    std::shared_ptr<BatchEvent> all;        // after the shared graphs' last work of a call
+    // an event of each call, after the shared graphs' last work, which those
+    // graphs hold until their next batched update
+    SpareRing<BatchEvent> events;
     BatchWorkers *workers = nullptr;
 };
 
@@ -2134,10 +2137,15 @@ lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *graphs, const
         // shared executors (host work, maybe an eager level-up), then the
         // rest, whose paths wait on the device, on several host threads
         std::vector<uint32_t> rest;
-        if (GS && !b->all) {
-            auto ev = std::make_shared<BatchEvent>();
-            CK(cudaEventCreateWithFlags(&ev->ev, cudaEventDisableTiming));
-            b->all = std::move(ev);
+        std::shared_ptr<BatchEvent> all;
+        if (GS) {
+            cudaError_t e = cudaSuccess;
+            all = b->events.take([&] {
+                auto x = std::make_shared<BatchEvent>();
+                e = cudaEventCreateWithFlags(&x->ev, cudaEventDisableTiming);
+                return e == cudaSuccess ? x : nullptr;
+            });
+            CK(e);
         }
         auto finish = [&](uint32_t k, cudaStream_t st) {
             const size_t i = forest[k];
@@ -2150,7 +2158,7 @@ lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *graphs, const
             h->front_sort_wide = false;  // the shared tile-merge sort
             h->front_part = false;
             res[i] = finish_update(h, rs, items[i].n_ins + items[i].n_del, 0, false, st, sts[i], &sts[i],
-                                   shared[k] != 0, false, shared[k] ? &b->all : nullptr);
+                                   shared[k] != 0, false, shared[k] ? &all : nullptr);
         };
         for (uint32_t k = 0; k < G; k++) {
             if (shared[k])
@@ -2158,7 +2166,7 @@ lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *graphs, const
             else
                 rest.push_back(k);
         }
-        if (GS) CK(cudaEventRecord(b->all->ev, s));
+        if (GS) CK(cudaEventRecord(all->ev, s));
         if (rest.size() > 1 && !prof_enabled()) {
             if (!b->workers) {
                 b->workers = new BatchWorkers();
