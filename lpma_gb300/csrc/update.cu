@@ -1731,16 +1731,19 @@ __global__ void __launch_bounds__(TPB) k_seg_update_counts(const UpdList u, uint
 // deletes(s) (its updates), and their exclusive prefixes PQ (the window
 // rank base of its items) and US (its first update), PQ[nseg] and
 // US[nseg] the totals.  The pairs are computed where they are read and
-// scanned packed in one u64 (each sum stays below 2^32): a reduce, a top
-// and a down pass.
+// scanned packed in one u64: a reduce, a top and a down pass.  Each half's
+// sum stays below 2^32, so none carries into the other: q is taken as 0
+// where it would be negative, which it is only for a segment of a small
+// window of the same loop, whose count holds the window's result while its
+// deletes are in the list still, and whose place in PQ is not read.
 constexpr uint32_t TS_IPT = 8, TS_TILE = TPB * TS_IPT;
 
 __device__ __forceinline__ uint64_t seg_pair(const uint8_t *__restrict__ cnt, const uint8_t *__restrict__ cnt_live,
                                              const uint32_t *__restrict__ qi, const uint32_t *__restrict__ qd,
                                              uint64_t s) {
     const uint32_t c = cnt_live ? cnt_live[s] : cnt[s];
-    const uint32_t i = qi[s], d = qd[s];
-    return (uint64_t)(c - d + i) | ((uint64_t)(i + d) << 32);
+    const uint32_t i = qi[s], d = qd[s], q = c + i > d ? c + i - d : 0u;
+    return (uint64_t)q | ((uint64_t)(i + d) << 32);
 }
 
 __global__ void __launch_bounds__(TPB) k_ts_reduce(const uint8_t *__restrict__ cnt, const uint8_t *__restrict__ cnt_live,
