@@ -330,7 +330,10 @@ typedef struct {
  * and, with unreachable set, waits for an arrival count that never comes,
  * so every wait gives up.  A sort whose wait gave up leaves the structure
  * unchanged and its update returns LPMA_ERR_TIMEOUT; the handle stays
- * usable.  Synchronous; no update may be in flight on the device. */
+ * usable.  The look-back of tier 5's digit passes polls as often, and not at
+ * all with unreachable set; its tiles then count for themselves, and the
+ * order is the same.
+ * Synchronous; no update may be in flight on the device. */
 LPMA_API lpma_status_t lpma_debug_sort_barrier(uint32_t poll_limit, int unreachable);
 
 /* Test setting of the executor of 5..32-segment windows on the current

@@ -263,10 +263,12 @@ __global__ void __launch_bounds__(256) k_hist(const uint64_t *__restrict__ keys,
 // A digit pass in one launch.  Tiles are handed out in order; a tile counts
 // its digits, publishes the counts, adds up those of the tiles before it (a
 // thread a digit, back to the nearest tile that has published its prefix)
-// while others do the same, publishes its own prefix and writes its keys.  A
-// tile waits only for lower ones, which are running and publish before they
-// wait; the wait is bounded all the same: after ONE_SPIN_LIMIT polls the sort
-// is marked as given up and the pass goes on, its writes within n.
+// while others do the same, publishes its own prefix and writes its keys
+// (the single-pass radix sort with decoupled look-back of Adinets and
+// Merrill).  A tile waits only for lower ones, which are running and publish
+// before they wait; the wait is bounded all the same: after ONE_SPIN_LIMIT
+// polls a thread counts its digit in the tiles before from their keys, which
+// a pass only reads, so the order is right whatever happens to the others.
 //
 // Bound by the ranking and the scatter, with HBM at half its rate.  One pass
 // over 16.8M keys: 154 us (160 with two CTAs an SM instead of three, 193 with
@@ -284,15 +286,26 @@ struct PassSmem {
     uint32_t gbase[256];  // place of the digit's first key of the tile, less ldig
     uint32_t ldig[256];
     uint32_t wsum[8];
-    uint32_t tile;
+    uint32_t tile, limit;
 };
+
+// The polls after which a thread counts.  Test setting (with the grid
+// barrier's): fewer, or 0, so that every thread counts at once.
+__device__ uint32_t g_one_limit = ONE_SPIN_LIMIT;
+
+// keys of digit d among the first n
+__device__ __forceinline__ uint32_t count_digit(const uint64_t *__restrict__ keys, uint64_t n, int sh, uint32_t d) {
+    uint32_t c = 0;
+    for (uint64_t p = 0; p < n; p++) c += (uint32_t)((keys[p] >> sh) & 0xFF) == d ? 1u : 0u;
+    return c;
+}
 
 // state: a word per digit of every tile, of this pass; cleared: the other
 // pass's, cleared here for the next one
 template <typename V>
 __global__ void __launch_bounds__(ONE_TPB, 3) k_onesweep(uint64_t *k0, V *v0, uint64_t *k1, V *v1, uint32_t n, int byte,
                                                       SortMask mask, const uint32_t *__restrict__ hist, uint32_t *state0,
-                                                      uint32_t *state1, uint32_t *next, uint32_t *err) {
+                                                      uint32_t *state1, uint32_t *next) {
     const uint32_t act = active_bytes(mask);
     if (!((act >> byte) & 1u)) return;
     const bool odd = __popc(act & ((1u << byte) - 1)) & 1;
@@ -306,7 +319,7 @@ __global__ void __launch_bounds__(ONE_TPB, 3) k_onesweep(uint64_t *k0, V *v0, ui
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PassSmem<V> &S = *reinterpret_cast<PassSmem<V> *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    if (tid == 0) S.tile = atomicAdd(&next[byte], 1u);
+    if (tid == 0) S.tile = atomicAdd(&next[byte], 1u), S.limit = g_one_limit;
     for (int i = tid; i < (ONE_TPB / 32) * 256; i += ONE_TPB) (&S.whist[0][0])[i] = 0;
     // exclusive sums over the digits (thread tid == digit, the upper half idle)
     auto digit_scan = [&](uint32_t x) {
@@ -373,7 +386,8 @@ __global__ void __launch_bounds__(ONE_TPB, 3) k_onesweep(uint64_t *k0, V *v0, ui
     if (tid < 256) {
         uint32_t before = 0, polls = 0;
         int64_t t = (int64_t)tile - 1;
-        while (t >= 0) {
+        bool lost = S.limit == 0;
+        while (t >= 0 && !lost) {
             uint32_t x[ONE_BACK];  // some tiles back at once
 #pragma unroll
             for (int q = 0; q < ONE_BACK; q++) x[q] = t >= q ? (uint32_t)state[(size_t)(t - q) * 256 + tid] : +ONE_PREFIX;
@@ -390,11 +404,9 @@ __global__ void __launch_bounds__(ONE_TPB, 3) k_onesweep(uint64_t *k0, V *v0, ui
                 }
             }
             if (done) break;
-            if (stuck && ++polls > ONE_SPIN_LIMIT) {
-                if (err) atomicOr(err, ERR_TIMEOUT);
-                break;
-            }
+            lost = stuck && ++polls >= S.limit;
         }
+        if (lost) before += count_digit(ko == k0 ? k1 : k0, (uint64_t)(t + 1) * ONE_TILE, 8 * byte, tid);
         if (tile) state[(size_t)tile * 256 + tid] = ((before + tcount) & ONE_VALUE) | ONE_PREFIX;
         S.gbase[tid] = dbase + before - S.ldig[tid];
     }
@@ -1394,7 +1406,7 @@ static cudaError_t sort_impl(uint64_t *k0, V *v0, uint64_t *k1, V *v1, uint32_t 
         if (!((mask.host_mask >> b) & 1u)) continue;
         ProfScope ps("sort_pass", st);
         k_onesweep<V><<<tiles, ONE_TPB, sm, st>>>(k0, v0, k1, v1, n, b, mask, s.hist + 256 * b, s.status,
-                                                  s.status + words, next, s.err);
+                                                  s.status + words, next);
         note_launch();
     }
     return cudaGetLastError();
@@ -1479,6 +1491,8 @@ static cudaError_t sort_setup_device(int dev, CoopCtas &out) {
 cudaError_t set_barrier_debug(uint32_t poll_limit, uint32_t unreachable) {
     cudaError_t e = cudaMemcpyToSymbol(g_bar_poll_limit, &poll_limit, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_bar_unreachable, &unreachable, sizeof(uint32_t));
+    const uint32_t limit = unreachable ? 0u : poll_limit ? poll_limit : ONE_SPIN_LIMIT;
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_one_limit, &limit, sizeof(uint32_t));
     return e;
 }
 

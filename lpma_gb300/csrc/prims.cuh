@@ -12,8 +12,8 @@ constexpr int SORT_TILE = SORT_TPB * SORT_IPT;  // 2048 keys per tile
 
 struct SortScratch {
     uint32_t *hist = nullptr;      // 8 x 256 global digit counts
-    uint32_t *status = nullptr;    // (digit, tile) counts and offsets of one pass
-    uint32_t *counters = nullptr;  // unused by the reduce-then-scan passes
+    uint32_t *status = nullptr;    // a word per digit of every tile, for two digit passes in turn
+    uint32_t *counters = nullptr;  // 16 words; 8 to 15: the tiles handed out by each digit pass
     size_t status_words = 0;
     // Set both to sort batches of up to coop_sort_max_keys() keys in one
     // cooperative launch: bar is a barrier counter word (cleared by the
@@ -138,15 +138,16 @@ cudaError_t sort_pairs_dev(uint64_t *k0, V *v0, uint64_t *k1, V *v1, uint32_t n,
 // Sorts n pairs by key (stable).  Only the bytes set in diff_bits are sorted
 // (bytes equal across all keys need no pass).  The result lands either in
 // (k0, v0) or in (k1, v1); *which receives 0 or 1.  err is kept for the
-// interface (no kernel of the sort waits on another CTA).
+// interface: the digit passes report no error (a tile whose wait for the ones
+// before it runs out counts their keys), the cooperative sort uses s.err.
 template <typename V>
 cudaError_t sort_pairs(uint64_t *k0, V *v0, uint64_t *k1, V *v1, uint32_t n, uint64_t diff_bits,
                        SortScratch &s, uint32_t *err, cudaStream_t st, int *which);
 
-// Status words needed for n keys: per-pass (digit, tile) counts and
-// offsets of the reduce-then-scan passes (tiles of SORT_TILE keys), or of
-// the cooperative sort (tiles of at least COOP_MIN_TILE keys, plus 256
-// digit totals), whichever is larger.
+// Status words needed for n keys: two words per digit and tile of SORT_TILE
+// keys (the digit passes, whose tiles are larger, use half of them), or the
+// cooperative sort's counts and offsets (tiles of at least COOP_MIN_TILE
+// keys, plus 256 digit totals), whichever is larger.
 constexpr int COOP_MIN_TILE = 1024;
 constexpr size_t sort_status_words(uint32_t n) {
     return (2 * (((size_t)n + SORT_TILE - 1) / SORT_TILE) * 256 + 2) >
@@ -167,7 +168,8 @@ constexpr size_t sort_status_words_wide(uint32_t n) {
 cudaError_t sort_prepare();
 
 // Test setting of the cooperative sort's grid barrier on the current device
-// (poll_limit 0: the default limit; unreachable: every wait gives up).
+// (poll_limit 0: the default limit; unreachable: every wait gives up) and of
+// the digit passes' look-back (with unreachable, every wait runs out).
 cudaError_t set_barrier_debug(uint32_t poll_limit, uint32_t unreachable);
 
 // Tile-merge sort of 16-bit-payload pairs: batches of TM_TILE_MAX + 1 ..
