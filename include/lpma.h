@@ -215,7 +215,11 @@ LPMA_API lpma_status_t lpma_destroy(LpmaHandle *h);
 LPMA_API const char *lpma_status_string(lpma_status_t s);
 
 /* ---- read paths: they read the structure in place (no CSR view is built)
- * and order after earlier work on `stream` (use the update stream). ---- */
+ * and order after earlier work on `stream` (use the update stream).  Reads
+ * of one handle on several streams, issued one after the other, are as on
+ * one: neighbour lists wait on the device for earlier ones, CSR views and
+ * PageRank for each other, since they share scratch of the handle.  Captured
+ * calls do not wait; run their graphs in order with the handle's reads. ---- */
 
 /* Replaces query_rpma(RPMA&, DEV_VEC_SIZE& srcs, DEV_VEC_KEY& constraints,
  * offset, len, edgelist, v_list) (rpma.cuh:1974-2036): for query i, the

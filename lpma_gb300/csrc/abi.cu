@@ -73,6 +73,14 @@ struct FrontGraph {
     cudaKernelNodeParams pack_params;
 };
 
+// Device scratch of a handle that a read still uses when its call returns: a
+// read of the same kind on another stream waits for it on the device.  A
+// captured call neither waits nor is waited for.
+struct ReadScratch {
+    cudaEvent_t ev = nullptr;
+    bool used = false;
+};
+
 struct BatchEvent {
     cudaEvent_t ev = nullptr;
     ~BatchEvent() {
@@ -149,6 +157,8 @@ struct LpmaHandle {
     // read paths (neighbour query, BFS, PageRank)
     NbrScratch q{};
     size_t q_cap = 0;
+    ReadScratch q_use;     // q
+    ReadScratch tile_use;  // c.segP and c.done (the views, a pulled PageRank)
     uint2 *bfs_a = nullptr, *bfs_b = nullptr;  // frontier lists
     uint32_t *bfs_cnt = nullptr;               // BFS_WORDS counters
     size_t bfs_cap = 0;
@@ -976,6 +986,22 @@ void mark_done(LpmaHandle *h, cudaStream_t s) {
     if (h->done_ev && cudaEventRecord(h->done_ev, s) == cudaSuccess) h->done_recorded = true;
 }
 
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+cudaError_t scratch_begin(const ReadScratch &u, cudaStream_t s) {
+    return u.used ? cudaStreamWaitEvent(s, u.ev, 0) : cudaSuccess;
+}
+
+cudaError_t scratch_end(ReadScratch &u, cudaStream_t s) {
+    cudaError_t e = u.ev ? cudaSuccess : cudaEventCreateWithFlags(&u.ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(u.ev, s);
+    u.used |= e == cudaSuccess;
+    return e;
+}
+
 // Polls the mirror's `published` word (set by the planner's last CTA after
 // the status words).  The front's event completes after the planner too:
 // queried now and then, it ends the wait with the error of a failed kernel,
@@ -1394,6 +1420,8 @@ lpma_status_t lpma_destroy(LpmaHandle *h) {
     // device-wide synchronisation, so other handles' streams keep running
     if (h->done_recorded) cudaEventSynchronize(h->done_ev);
     if (h->batch_done) cudaEventSynchronize(h->batch_done->ev);
+    for (const ReadScratch *u : {&h->q_use, &h->tile_use})
+        if (u->used) cudaEventSynchronize(u->ev);
     for (cudaStream_t st : {h->side_stream, h->cap_stream, h->copy_stream})
         if (st) cudaStreamSynchronize(st);
     for (FrontGraph &f : h->graphs) {
@@ -1429,6 +1457,8 @@ lpma_status_t lpma_destroy(LpmaHandle *h) {
         dfree_async(h->bfs_cnt);
     dfree_async(h->pr_deg), dfree_async(h->pr_contrib), dfree_async(h->pr_acc), dfree_async(h->pr_dangling);
     if (h->done_ev) cudaEventDestroy(h->done_ev);
+    for (const ReadScratch *u : {&h->q_use, &h->tile_use})
+        if (u->ev) cudaEventDestroy(u->ev);
     pinned_release(h->pin_word, PIN_WORDS * sizeof(uint32_t));
     delete h;
     return LPMA_OK;
@@ -1620,9 +1650,12 @@ static lpma_status_t fill_view(LpmaHandle *h, cudaStream_t s, bool csr, bool exp
         h->exp_cap = nnz + 1;
     }
     Geo g{h->c.keys, h->c.vals, h->H};
+    const bool cap = capturing(s);
+    if (!cap) CK(scratch_begin(h->tile_use, s));
     launch_csr_fill(g, h->c.cnt, h->c.segP, h->c.done, csr ? h->row_offset : nullptr, csr ? h->col_index : nullptr,
                     csr ? h->view_vals : nullptr, exp ? h->exp_keys : nullptr, exp ? h->exp_vals : nullptr, s);
     CK(cudaGetLastError());
+    if (!cap) CK(scratch_end(h->tile_use, s));
     return LPMA_OK;
 }
 
@@ -1758,6 +1791,7 @@ lpma_status_t lpma_query_neighbors(LpmaHandle *h, const uint32_t *d_srcs, const 
     }
     Geo g{h->c.keys, h->c.vals, h->H};
     if (n) {
+        CK(scratch_begin(h->q_use, s));
         CK(launch_nbr_count(d_srcs, d_windows, (uint32_t)n, g, h->c.cnt, h->sent, h->V, h->q, d_offsets, s));
     } else {
         CK(cudaMemsetAsync(d_offsets, 0, sizeof(uint32_t), s));
@@ -1769,7 +1803,7 @@ lpma_status_t lpma_query_neighbors(LpmaHandle *h, const uint32_t *d_srcs, const 
     if (*total > cap) return LPMA_ERR_BUFFER_TOO_SMALL;
     launch_nbr_fill(d_srcs, d_windows, (uint32_t)n, g, h->c.cnt, h->sent, h->V, h->q, d_nbrs, d_vals, s);
     CK(cudaGetLastError());
-    mark_done(h, s);
+    CK(scratch_end(h->q_use, s));  // lpma_destroy waits for it as for the done event
     return LPMA_OK;
 }
 
@@ -1851,9 +1885,7 @@ lpma_status_t lpma_pagerank(LpmaHandle *h, double alpha, uint32_t iterations, do
     }
     const Geo g{h->c.keys, h->c.vals, h->H};
     // (a captured call allocates nothing and pushes)
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(s, &cs));
-    if (cs == cudaStreamCaptureStatusNone && pagerank_pulls(h->total - h->V, iterations)) {
+    if (!capturing(s) && pagerank_pulls(h->total - h->V, iterations)) {
         // the edges by destination and the reciprocal degrees, for this call
         PrLayout l;
         const uint64_t words = pr_words(h->V, h->total - h->V, &l);
@@ -1864,8 +1896,10 @@ lpma_status_t lpma_pagerank(LpmaHandle *h, double alpha, uint32_t iterations, do
             uint32_t *w = static_cast<uint32_t *>(mem);
             double2 *inv = reinterpret_cast<double2 *>(static_cast<char *>(mem) + at);
             const uint64_t nseg = nseg_of(h->H);
-            cudaError_t x = scan_u8_to_u32(h->c.cnt, h->c.segP, (uint32_t)nseg, h->c.segP + nseg, h->c.scan_tmp, s);
+            cudaError_t x = scratch_begin(h->tile_use, s);
+            if (!x) x = scan_u8_to_u32(h->c.cnt, h->c.segP, (uint32_t)nseg, h->c.segP + nseg, h->c.scan_tmp, s);
             if (!x) x = launch_pr_layout(g, h->c.cnt, h->c.segP, h->sent, h->V, l, w, inv, s);
+            if (!x) x = scratch_end(h->tile_use, s);
             if (!x) x = cudaMemsetAsync(h->pr_dangling, 0, 3 * sizeof(double), s);
             for (uint32_t it = 0; it <= iterations && !x; it++)
                 launch_pr_pull(it, l, w, h->V, alpha, inv, d_rank, h->pr_contrib, h->pr_acc, h->pr_dangling,
