@@ -12,12 +12,12 @@
 //
 // One update: the keys validated and partitioned by the upper levels of the
 // locate's descent, each bucket ordered and resolved by one CTA (batches of
-// more than 2^20 keys, small trees and batches that crowd into one bucket:
-// pack, the shared radix sort, resolve): locate by binary search over the
-// first slot of each segment, membership scan of the segment, upsert /
-// tombstone / a tombstoned key brought back in place; the pending inserts
-// laid end to end as the update list, then the shared
-// count-only planner and maximal-window filter (k_plan / k_plan_max, with
+// more than 2^20 keys, small trees, batches that crowd into one bucket or
+// whose buckets find no memory: pack, the shared radix sort, resolve):
+// locate by binary search over the first slot of each segment, membership
+// scan of the segment, upsert / tombstone / a tombstoned key brought back in
+// place; the pending inserts laid end to end as the update list, then the
+// shared count-only planner and maximal-window filter (k_plan / k_plan_max, with
 // the flat segment length and count) over per-segment live counts.  The
 // maximal windows run on flat executors: single-segment windows a group of
 // lanes each, windows of up to 32 segments one CTA each in shared memory, bigger
@@ -836,7 +836,7 @@ struct GpmaState {
     uint32_t *row = nullptr;  // V + 1
     DevStatus *dst = nullptr, *hst = nullptr;
     uint32_t sticky = 0;
-    uint32_t part_skip = 0;  // batches left that the sorted front takes, after a bucket overflowed
+    uint32_t part_skip = 0;  // batches left that the sorted front takes, after a bucket overflowed or found no room
 };
 
 namespace {
@@ -1018,8 +1018,9 @@ void gpma_part_plan(const GpmaState *g, uint64_t n, uint32_t *L, uint32_t *cap) 
 }
 
 // One update through the partitioned front, with one host round trip unless
-// it has big windows or rebuilds; *done is false when a bucket overflowed
-// and nothing was changed.
+// it has big windows or rebuilds; *done is false when a bucket overflowed or
+// there is no room for the buckets (the sorted front takes its memory in
+// pieces), and nothing was changed.
 lpma_status_t update_part(GpmaState *g, const uint64_t *ins, const uint8_t *ins_vals, uint32_t n_ins, const uint64_t *del,
                           uint32_t n_del, uint32_t L, uint32_t cap, cudaStream_t s, LpmaStats &st, bool *done) {
     *done = true;
@@ -1052,7 +1053,15 @@ lpma_status_t update_part(GpmaState *g, const uint64_t *ins, const uint8_t *ins_
             part(&u.key, k), part(&u.val, k), part(&u.kind, k), part(&u.seg, k), part(&u.ip, k + 1), part(&pend, k);
             part(&wl, 5 * k), part(&P, nseg + 1), part(&tmp, scan_tmp_words((uint32_t)nseg) + 64);
         }
-        if (!pass) GCK(salloc(&arena, off, s));
+        if (!pass) {
+            const cudaError_t e = salloc(&arena, off, s);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                *done = false;
+                return LPMA_OK;
+            }
+            GCK(e);
+        }
     }
     struct Release {
         uint8_t *&p;
