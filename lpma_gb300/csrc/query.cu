@@ -6,6 +6,7 @@
 
 #include "kernels.cuh"
 #include "prims.cuh"
+#include "quotient.h"
 
 namespace lpma {
 namespace {
@@ -767,8 +768,10 @@ __global__ void __launch_bounds__(TPB) k_pr_deg(const uint32_t *__restrict__ P, 
 // (base = (1 - alpha) / V, first = 1 / V).
 //
 // Bound by the FP64 pipes, which take two lanes a clock: five operations a
-// vertex, the degree being stored as a double beside its reciprocal.  So no thread divides (three quotients a thread took 20 of the
-// 28 us of a step over 1M vertices), and zero sums are not added up.
+// vertex, the degree being stored as a double beside its reciprocal.  So no
+// thread divides (three quotients a thread took 20 of the 28 us of a step
+// over 1M vertices; quotient.h has the same result), and zero sums are not
+// added up.
 __global__ void __launch_bounds__(TPB) k_pr_step(bool init, double *rank, double *acc, const double2 *__restrict__ inv,
                                                  uint32_t V, double alpha, double base, double first, const double *__restrict__ dangling, double *next,
                                                  double *after, double *contrib) {
@@ -786,10 +789,7 @@ __global__ void __launch_bounds__(TPB) k_pr_step(bool init, double *rank, double
             contrib[v] = 0.0;
             d += r;
         } else {
-            // rank / deg from the rounded reciprocal: one correction step
-            // gives the quotient's rounding
-            const double q = r * i.x;
-            contrib[v] = fma(fma(-q, i.y, r), i.x, q);
+            contrib[v] = quotient(r, i.y, i.x);  // alpha is at most 1: no rank is infinite
         }
     }
     if (__any_sync(0xffffffffu, __double_as_longlong(d) != 0))
