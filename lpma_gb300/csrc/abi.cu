@@ -79,6 +79,7 @@ struct FrontGraph {
 struct ReadScratch {
     cudaEvent_t ev = nullptr;
     bool used = false;
+    unsigned long long stream = 0;  // the id of the stream of the last use (no other stream ever has it)
 };
 
 struct BatchEvent {
@@ -992,11 +993,15 @@ bool capturing(cudaStream_t s) {
 }
 
 cudaError_t scratch_begin(const ReadScratch &u, cudaStream_t s) {
-    return u.used ? cudaStreamWaitEvent(s, u.ev, 0) : cudaSuccess;
+    unsigned long long id = 0;
+    if (!u.used || (cudaStreamGetId(s, &id) == cudaSuccess && id == u.stream)) return cudaSuccess;
+    return cudaStreamWaitEvent(s, u.ev, 0);
 }
 
+// lpma_destroy waits for the use, as for the done event
 cudaError_t scratch_end(ReadScratch &u, cudaStream_t s) {
     cudaError_t e = u.ev ? cudaSuccess : cudaEventCreateWithFlags(&u.ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamGetId(s, &u.stream);
     if (e == cudaSuccess) e = cudaEventRecord(u.ev, s);
     u.used |= e == cudaSuccess;
     return e;
@@ -1655,7 +1660,10 @@ static lpma_status_t fill_view(LpmaHandle *h, cudaStream_t s, bool csr, bool exp
     launch_csr_fill(g, h->c.cnt, h->c.segP, h->c.done, csr ? h->row_offset : nullptr, csr ? h->col_index : nullptr,
                     csr ? h->view_vals : nullptr, exp ? h->exp_keys : nullptr, exp ? h->exp_vals : nullptr, s);
     CK(cudaGetLastError());
-    if (!cap) CK(scratch_end(h->tile_use, s));
+    if (cap)
+        mark_done(h, s);
+    else
+        CK(scratch_end(h->tile_use, s));
     return LPMA_OK;
 }
 
@@ -1668,7 +1676,6 @@ lpma_status_t lpma_csr_view(LpmaHandle *h, const uint32_t **row_offset, const ui
     if (!h->view_valid) {
         CKS(fill_view(h, s, true, false));
         h->view_valid = true;
-        mark_done(h, s);
     }
     *row_offset = h->row_offset;
     *col_index = h->col_index;
@@ -1803,7 +1810,7 @@ lpma_status_t lpma_query_neighbors(LpmaHandle *h, const uint32_t *d_srcs, const 
     if (*total > cap) return LPMA_ERR_BUFFER_TOO_SMALL;
     launch_nbr_fill(d_srcs, d_windows, (uint32_t)n, g, h->c.cnt, h->sent, h->V, h->q, d_nbrs, d_vals, s);
     CK(cudaGetLastError());
-    CK(scratch_end(h->q_use, s));  // lpma_destroy waits for it as for the done event
+    CK(scratch_end(h->q_use, s));
     return LPMA_OK;
 }
 
