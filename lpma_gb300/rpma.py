@@ -9,6 +9,7 @@ implementation behind this module.
 """
 import ctypes
 from array import array
+from itertools import islice
 
 import numpy as np
 
@@ -406,19 +407,20 @@ class Batcher:
         # struct field at a time, 415 so (240 of them in the tensors' own calls)
         words = array("Q")
         keep = []  # the words hold addresses: an iterator's batches live in here until the call returns
-        for _, b in zip(graphs, batches):
+        for b in islice(batches, n):
             if not isinstance(b, dict):
                 b = {"ins": b[0], "dels": b[1]}
+            keep.append(b)
             ins, vals, dels = b.get("ins"), b.get("ins_vals"), b.get("dels")
-            keep.append((ins, vals, dels))
             pi, ni = _dev(ins, "uint64") if ins is not None else (0, 0)
             pd, nd = _dev(dels, "uint64") if dels is not None else (0, 0)
             words.extend((pi, _dev(vals, "uint8")[0] if vals is not None else 0, ni, pd, nd,
                           int(b.get("thres", 0)) & 0xFFFFFFFF))
         # a graph without a batch is refused: it gets no handle
-        words.extend([0] * (6 * n - len(words)))
-        hs = array("Q", [g._h.value or 0 for g, _ in zip(graphs, keep)])
-        hs.extend([0] * (n - len(hs)))
+        m = len(keep)
+        words.extend([0] * (6 * (n - m)))
+        hs = array("Q", [g._h.value or 0 for g in graphs])
+        hs[m:] = array("Q", [0] * (n - m))
         stats = (LpmaStats * n)()
         status = (ctypes.c_int * n)()
         rc = self._L.lpma_update_batch(self._b, hs.buffer_info()[0], words.buffer_info()[0], n, _stream_ptr(stream), stats,
