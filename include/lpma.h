@@ -252,7 +252,7 @@ LPMA_API lpma_status_t lpma_edge_query(LpmaHandle *h, const uint64_t *d_keys, si
  * unreached (nvGRAPH's convention).  max_depth bounds the levels (0: no
  * bound; 2 for a 2-hop BFS from many seeds).  levels / reached (may be
  * NULL) receive the levels expanded and the vertices reached.  Synchronises
- * once per level. */
+ * once per four levels. */
 LPMA_API lpma_status_t lpma_bfs(LpmaHandle *h, const uint32_t *d_sources, size_t n_sources, uint32_t max_depth,
                                 int32_t *d_dist, uint32_t *levels, uint64_t *reached, lpma_stream_t stream);
 
@@ -302,11 +302,12 @@ LPMA_API lpma_status_t lpma_update_batch(LpmaBatcher *b, LpmaHandle *const *grap
                                          size_t n, lpma_stream_t stream, LpmaStats *stats, lpma_status_t *status);
 
 /* ---- autotuner: the batch-sort algorithm per batch-size bucket ----
- * Batches of 256 to 2^21 keys, no more than are stored, on trees of height 9 and more take the
- * partitioned front, which does not sort the whole batch, unless they
- * crowd into one of its buckets; lpma_tune_set with a tier other than 0
- * keeps the batches of its entry off it.  The sorted front sorts each batch
- * with one of five algorithms ("tiers"):
+ * Batches of 256 to 2^21 keys, no more than are stored, on trees of height
+ * 9 and more take the partitioned front, which does not sort the whole
+ * batch, unless they crowd into one of its buckets; lpma_tune_set with a
+ * tier other than 0 keeps the batches of its entry off it, which is slower
+ * for most (set 0 again to undo it; what lpma_autotune keeps does not).  The
+ * sorted front sorts each batch with one of five algorithms ("tiers"):
  * 1 one CTA through shared memory (<= 2048 keys), 2 tiles of 2048 keys
  * sorted by all-pairs rank over many CTAs, then placed by binary searches
  * across the tiles (<= 16384), 3 register-sorted tiles plus

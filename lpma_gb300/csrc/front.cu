@@ -15,9 +15,8 @@
 // the same items.
 //
 // What bounds it: the partition, the scatter of 16-byte entries into L2; the
-// buckets, instructions (about 100 a key; 57% of the issue slots, HBM at a
-// third of its rate): the segments are asked of L2 while the CTA orders its
-// keys.  A batch of 1M keys into a scale-21 graph: partition 29 us, buckets
+// buckets, instructions (95 a key; 59% of the issue slots, HBM at 24% of its
+// rate): the segments are asked of L2 while the CTA orders its keys.  A batch of 1M keys into a scale-21 graph: partition 29 us, buckets
 // 139, list 8, and the planner 20 on the 5% of the segments that remain;
 // before, pack 17, sort 87, locate 46, compaction 18, planner 51, executor 89.
 #include <algorithm>

@@ -2070,16 +2070,18 @@ __global__ void __launch_bounds__(GT_TPB) k_spread(const TileJob *__restrict__ j
 
 // ------------------------------------------------------------------ respread
 // The whole array (a root window, or a rebuild at another height) goes from
-// one slot array to another in one pass.  A CTA takes 128 destination
-// segments, so at most 4,096 ranks, finds the source segments that hold
-// them, merges their kept slots and inserts in shared memory in rank order
-// and writes its segments whole.
+// one slot array to another in one pass.  A CTA takes a run of destination
+// segments (launch_respread: as many as 4,096 items fill and as 7 source
+// tiles feed, 224 at equal heights), finds the source segments that hold
+// their items, merges the kept slots and inserts in shared memory in rank
+// order and writes its segments whole.
 //
 // It reads the occupied slots once and writes all slots once; gather and
 // spread write and read a contiguous copy in between, after counts per
 // segment, a scan of them and a sorted job list.  Bound by instructions (the
-// merge of four segments a warp takes about 350; half of the issue slots)
-// and the chain of dependent reads from the rank to the slots; HBM is at 30%.
+// merge of four segments a warp takes about 350; 43% of the issue slots in a
+// rebuild of 1M segments at the next height) and the chain of dependent reads
+// from the rank to the slots; HBM is at a fifth of its rate.
 // 15.2M items and 1M updates over 1M segments: 165 us and 12 for the tiles'
 // prefixes (258 us before).  With 128 destination segments a CTA it took 240
 // (4 or 5 of the 8 warps had a tile), with 256 190 (a ninth tile).
